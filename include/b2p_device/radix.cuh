@@ -17,14 +17,11 @@
 //   * spine: per digit, an exclusive scan of its counts over the chunks and
 //     its total; a digit's first slot in chunk b is then the keys of smaller
 //     digits plus the keys of that digit in chunks before b;
-//   * downsweep: block b walks its chunk's tiles in order.  Its warps rank
-//     each tile's keys in key order (warp w owns 32 consecutive keys per
-//     round; lanes holding the same digit find each other with one ballot
-//     per digit bit, and a per-warp count per digit gives each key its
-//     rank), the keys are
-//     reordered by digit in shared memory, written to their slots (running
-//     slot of the digit + position in the tile's run of that digit), and the
-//     running slots advance by the tile's counts.
+//   * downsweep: block b walks its chunk's tiles in order, ranks each tile's
+//     keys in key order, reorders the tile by digit in shared memory and
+//     writes the keys to their slots (running slot of the digit + position in
+//     the tile's run of that digit); the running slots advance by the tile's
+//     counts.
 // Nothing waits on another block, and the sort is stable: chunks, tiles and
 // keys inside a tile are taken in index order.
 #pragma once
@@ -32,42 +29,26 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <limits>
 
 namespace b2p {
 
 constexpr int kRadixBits = 8, kRadixBins = 1 << kRadixBits;
+// upsweep blocks
 constexpr int kRadixThreads = 256, kRadixItems = 16;
-constexpr int kRadixTile = kRadixThreads * kRadixItems;  // 4096 keys
-constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kRadixBlocksPerSm = 4;
+constexpr int kRadixStep = kRadixThreads * kRadixItems;  // 4096 keys
+// downsweep blocks
+constexpr int kDownThreads = 128;
+constexpr int kRadixItemBytes = 256;                             // keys of one thread
+constexpr int kRadixTileBytes = kDownThreads * kRadixItemBytes;  // 32 KiB
+constexpr int kDownBlocksPerSm = 3;                              // 2 x 32 KiB of shared memory each
+template <class T>
+constexpr long long radix_tile() {
+  return kRadixTileBytes / (long long)sizeof(T);
+}
 constexpr int kRadixSpineThreads = 1024;
 // 32-bit slots: inputs below 2^31 keys
 constexpr size_t kRadixMaxKeys = (size_t)1 << 31;
-
-template <class T>
-struct RadixKey {
-  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4- or 8-byte keys");
-  using U = typename std::conditional<sizeof(T) == 4, unsigned, unsigned long long>::type;
-  static constexpr int kPasses = (int)sizeof(T) * 8 / kRadixBits;
-  static constexpr U kSign = (U)1 << (sizeof(T) * 8 - 1);
-  __device__ __forceinline__ static U order(const T &x, bool desc) {
-    U u;
-    memcpy(&u, &x, sizeof(T));
-    U k;
-    if constexpr (std::is_floating_point<T>::value) {
-      if (u == kSign) u = 0;  // -0.0 == +0.0
-      k = (u & kSign) ? (U)~u : (U)(u | kSign);
-    } else if constexpr (std::is_signed<T>::value) {
-      k = u ^ kSign;
-    } else {
-      k = u;
-    }
-    return desc ? (U)~k : k;
-  }
-  __device__ __forceinline__ static unsigned digit(const T &x, bool desc, int pass) {
-    return (unsigned)(order(x, desc) >> (pass * kRadixBits)) & (kRadixBins - 1);
-  }
-};
 
 // Scratch of a radix sort of n keys of T with `blocks` persistent blocks:
 // the per-chunk digit counts (then their prefixes), the digit totals and the
@@ -83,8 +64,8 @@ template <class T>
 inline RadixLayout radix_layout(size_t n, int sm_count) {
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   RadixLayout l;
-  l.ntiles = (long long)((n + kRadixTile - 1) / kRadixTile);
-  const long long want = (long long)std::max(sm_count, 1) * kRadixBlocksPerSm;
+  l.ntiles = ((long long)n + radix_tile<T>() - 1) / radix_tile<T>();
+  const long long want = (long long)std::max(sm_count, 1) * kDownBlocksPerSm;
   l.chunk = (l.ntiles + want - 1) / want;
   l.blocks = (int)((l.ntiles + l.chunk - 1) / l.chunk);
   l.counts = kHeaderBytes;
@@ -101,50 +82,88 @@ inline size_t radix_scratch_bytes(size_t n) {
   return radix_layout<T>(n, 256).total + 256;
 }
 
-// Lanes of the warp whose label (a digit, or 256 for a key past the end)
-// equals this lane's: one ballot per label bit (BITS = 8 when every key of
-// the round is real, 9 otherwise).
-template <int BITS>
-__device__ __forceinline__ unsigned radix_peers(unsigned label) {
-  unsigned peers = 0xffffffffu;
-#pragma unroll
-  for (int b = 0; b < BITS; ++b) {
-    const bool bit = (label >> b) & 1u;
-    const unsigned m = __ballot_sync(0xffffffffu, bit);
-    peers &= bit ? m : ~m;
+// Digit `pass` of a key under the key order.  A key's order digit is its own
+// digit, xored with a constant of the pass (the sign bit, the complement of a
+// descending sort) and, for floats, with the sign of the key.
+template <class T>
+struct RadixDigit {
+  static constexpr bool kFloat = std::is_floating_point<T>::value;
+  static constexpr int kLast = (int)sizeof(T) - 1;
+  unsigned place, flip, top;
+  bool high;
+  __device__ __forceinline__ RadixDigit(int pass, bool desc)
+      : place(8u * (pass & 3)),
+        flip((desc ? 0xffu : 0u) ^ (std::is_integral<T>::value && std::is_signed<T>::value && pass == kLast ? 0x80u : 0u)),
+        top(kFloat && pass == kLast ? 0x80u : 0u),
+        high(pass >= 4) {}
+  // (digit << SHIFT) ^ c
+  template <int SHIFT>
+  __device__ __forceinline__ unsigned at(const T &x, unsigned c) const {
+    constexpr unsigned M = 0xffu << SHIFT;
+    unsigned w, sign = 0;
+    if constexpr (sizeof(T) == 4) {
+      memcpy(&w, &x, 4);
+      if constexpr (kFloat) {
+        if (w == 0x80000000u) w = 0;  // -0.0 == +0.0
+        sign = (unsigned)((int)w >> 31);
+      }
+    } else {
+      uint2 v;
+      memcpy(&v, &x, 8);
+      if constexpr (kFloat) {
+        if (v.y == 0x80000000u && v.x == 0) v.y = 0;
+        sign = (unsigned)((int)v.y >> 31);
+      }
+      w = high ? v.y : v.x;
+    }
+    unsigned r = __funnelshift_r(w, w, (place - SHIFT) & 31u) & M;
+    if constexpr (kFloat) r ^= (sign & M) | (top << SHIFT);
+    return r ^ (c ^ (flip << SHIFT));
   }
-  return peers;
-}
+};
 
 // Upsweep: digit counts of block b's chunk of tiles, counts[d * blocks + b].
+// Counter (digit, lane) is word digit * 32 + lane, one for the lanes of that
+// number in all warps: a warp's 32 atomics lie in 32 different banks.  Bound
+// by the read: 2^28 int32 keys take 185 us (5.8 TB/s); one counter per digit
+// and warp, with its bank conflicts and scalar loads, took 209 us.
 template <class T>
-__global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *keys, size_t n, bool desc, int pass,
+__global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *keys, unsigned n, bool desc, int pass,
                                                                     long long chunk, unsigned *counts) {
-  __shared__ unsigned sh[kRadixWarps][kRadixBins];  // one histogram per warp
-  for (int i = threadIdx.x; i < kRadixWarps * kRadixBins; i += kRadixThreads) (&sh[0][0])[i] = 0;
+  __shared__ __align__(16) unsigned sh[kRadixBins * 32];
+  constexpr unsigned IPV = 16 / sizeof(T), V = kRadixItems / IPV;
+  const unsigned t = threadIdx.x, lane = t & 31u;
+  for (unsigned i = t; i < kRadixBins * 8; i += kRadixThreads)
+    reinterpret_cast<uint4 *>(sh)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  unsigned *wsh = sh[threadIdx.x >> 5];
-  const size_t b0 = (size_t)blockIdx.x * chunk * kRadixTile;
-  const size_t b1 = min(n, b0 + (size_t)chunk * kRadixTile);
-  // a tile at a time, every thread's kRadixItems loads in flight together
-  for (size_t base = b0; base < b1; base += kRadixTile) {
-    T key[kRadixItems];
+  const RadixDigit<T> dg(pass, desc);
+  auto count = [&](const T &k) {
+    atomicAdd(reinterpret_cast<unsigned *>(reinterpret_cast<char *>(sh) + dg.template at<7>(k, lane << 2)), 1u);
+  };
+  const unsigned b0 = (unsigned)(blockIdx.x * chunk * radix_tile<T>());
+  const unsigned b1 = (unsigned)min((long long)n, b0 + chunk * radix_tile<T>());
+  unsigned i = b0;
+  if ((reinterpret_cast<uintptr_t>(keys) & 15) == 0) {
+    // every thread's V 16-byte loads in flight together
+    for (; i + kRadixStep <= b1; i += kRadixStep) {
+      uint4 v[V];
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
-      const size_t i = base + (size_t)r * kRadixThreads + threadIdx.x;
-      if (i < b1) key[r] = keys[i];
-    }
+      for (unsigned r = 0; r < V; ++r) v[r] = ld_stream_v4(keys + i + (r * kRadixThreads + t) * IPV);
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
-      const size_t i = base + (size_t)r * kRadixThreads + threadIdx.x;
-      if (i < b1) atomicAdd(&wsh[RadixKey<T>::digit(key[r], desc, pass)], 1u);
+      for (unsigned r = 0; r < V; ++r) {
+        T k[IPV];
+        memcpy(k, &v[r], 16);
+#pragma unroll
+        for (unsigned e = 0; e < IPV; ++e) count(k[e]);
+      }
     }
   }
+  for (i += t; i < b1; i += kRadixThreads) count(keys[i]);
   __syncthreads();
-  for (int d = threadIdx.x; d < kRadixBins; d += kRadixThreads) {
+  for (unsigned d = t; d < kRadixBins; d += kRadixThreads) {
     unsigned c = 0;
 #pragma unroll
-    for (int w = 0; w < kRadixWarps; ++w) c += sh[w][d];
+    for (unsigned r = 0; r < 32; ++r) c += sh[d * 32 + ((r + d) & 31u)];
     counts[(size_t)d * gridDim.x + blockIdx.x] = c;
   }
 }
@@ -172,141 +191,299 @@ __global__ void __launch_bounds__(kRadixSpineThreads) radix_spine_kernel(unsigne
   if (t == kRadixSpineThreads - 1) totals[blockIdx.x] = before + incl;
 }
 
-// Dynamic shared memory of radix_downsweep_kernel<T>: the tile's keys,
-// per-warp digit counts (257 buckets: 256 = past the end), the tile's
-// counts, the running output slots and the tile-local digit starts.
+// ------------------------------------------------------------- downsweep
+//
+// Ranking.  Every thread owns kRadixItemBytes / sizeof(T) consecutive keys of
+// the tile and its own 8-bit counter of every digit.  Counter (digit, thread)
+// is byte `warp` of word digit * 32 + lane, so a warp's 32 counters of any 32
+// digits lie in 32 different banks: one shared atomicAdd per key, one
+// wavefront per warp whatever the digits are, returns the key's rank among
+// the thread's keys of its digit.  A word holds the four threads (one of each
+// warp) that own neighbouring key blocks: thread (warp, lane) owns block
+// 4 * lane + warp.
+//
+// The prefix of the counters along the key order is a product with a
+// triangular matrix of ones, taken by integer mma.sync straight from the
+// counter words: row = digit, k = the bytes of the 32 words, column = word,
+// giving for every word the keys of the digit up to and with it.  The bytes
+// of the word from the thread's own on are taken off again with one dp4a.
+//
+// Bound by shared-memory wavefronts: 14.4 per 32 keys (4.2 of them the
+// scatter into the sorted tile, whose banks are random), the data pipe 73 %
+// busy at 2^26 keys.  2^28 random int32 keys: 670 us a pass; ranking by eight
+// ballots per key, 118 instructions per 32 keys, took 1,525 us.  64 keys a
+// thread halve the counters' clearing and prefix work per key against 32.
+// Three blocks of 128 threads is what 2 x 32 KiB each leaves room for; the
+// keys stay in registers (168 per thread) from the count to the scatter.
+
+// D += A * B, 16 digits x 8 words, k = 32 counter bytes.
+__device__ __forceinline__ void radix_mma(int (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
+                                          unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Byte offset of 16-byte chunk c of thread row r in the staged tile: rows of
+// 256 bytes, chunks swizzled so that neighbouring rows' equal chunks lie in
+// different banks.
+__device__ __forceinline__ unsigned radix_stage(unsigned r, unsigned c) {
+  return r * kRadixItemBytes + ((c ^ (r & 15u)) << 4);
+}
+
+// Bring tile `t0 .. t0 + count` of `in` into `buf`, block kb in row
+// (kb & 3) * 32 + kb / 4; keys past the end are `pad` (digit 255 in every
+// pass, so that they stay behind the tile's real keys).  Full tiles of
+// 16-byte aligned input come by cp.async.
+template <class T>
+__device__ __forceinline__ void radix_load_tile(char *buf, const T *in, unsigned t0, unsigned count, bool vec, T pad) {
+  constexpr unsigned K = kRadixItemBytes / sizeof(T), TILE = K * kDownThreads;
+  const unsigned t = threadIdx.x;
+  if (vec && count == TILE) {
+    const char *g = reinterpret_cast<const char *>(in + t0) + t * 16;
+    const unsigned c = t & 15u, row0 = ((t >> 4) & 3u) * 32u + (t >> 6);
+#pragma unroll
+    for (unsigned q = 0; q < 16; ++q) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(buf + radix_stage(row0 + 2 * q, c));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g + (size_t)q * kDownThreads * 16)
+                   : "memory");
+    }
+  } else {
+    for (unsigned e = t; e < TILE; e += kDownThreads) {
+      const unsigned kb = e / K, b = (e % K) * (unsigned)sizeof(T);
+      const T x = e < count ? in[t0 + e] : pad;
+      *reinterpret_cast<T *>(buf + radix_stage((kb & 3u) * 32u + (kb >> 2), b >> 4) + (b & 15u)) = x;
+    }
+  }
+}
+
 template <class T>
 constexpr size_t radix_pass_smem() {
-  return sizeof(T) * kRadixTile + sizeof(unsigned) * (kRadixWarps * (kRadixBins + 1) + 3 * kRadixBins);
+  return 2 * (size_t)kRadixTileBytes;
 }
 
 // Downsweep: block b moves its chunk's keys from `in` to their slots in
 // `out` by digit `pass`, tile by tile; prefix[d * blocks + b] counts digit d
 // in the chunks before b, totals[d] in the whole input (the spine's results).
+//
+// Two 32 KiB buffers change places from tile to tile: x holds the staged
+// keys, then (the keys being in registers) the prefixes, then the tile sorted
+// by digit; y holds the counters, then the next tile on its way in.
 template <class T>
-__global__ void __launch_bounds__(kRadixThreads, kRadixBlocksPerSm)
-    radix_downsweep_kernel(const T *in, T *out, size_t n, bool desc, int pass, long long chunk,
-                           const unsigned *prefix, const unsigned *totals) {
-  extern __shared__ __align__(16) unsigned char radix_smem[];
-  T *s_keys = reinterpret_cast<T *>(radix_smem);
-  unsigned *s_wh = reinterpret_cast<unsigned *>(radix_smem + sizeof(T) * kRadixTile);
-  unsigned *s_tot = s_wh + kRadixWarps * (kRadixBins + 1);
-  unsigned *s_run = s_tot + kRadixBins;
-  unsigned *s_lstart = s_run + kRadixBins;
-  __shared__ unsigned s_scan[kRadixBins / 32];
+__global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
+    radix_downsweep_kernel(const T *in, T *out, unsigned n, bool desc, int pass, long long chunk,
+                           const unsigned *prefix, const unsigned *totals, T pad) {
+  constexpr unsigned S = sizeof(T), K = kRadixItemBytes / S, TILE = K * kDownThreads;
+  static_assert(K <= 64, "a word's four counters stay below 256 and signed");
+  extern __shared__ __align__(128) unsigned char radix_smem[];
+  __shared__ __align__(16) unsigned s_tot[kRadixBins], s_start[kRadixBins], s_base[kRadixBins];
+  char *x = reinterpret_cast<char *>(radix_smem), *y = x + kRadixTileBytes;
 
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  {
-    // first slot of digit t for this chunk: keys of smaller digits (an
-    // exclusive scan of the digit totals) + keys of digit t in earlier chunks
-    const unsigned c = totals[t];
-    unsigned incl = c;
+  const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  const RadixDigit<T> dg(pass, desc);
+  auto counter = [&](const T &k) { return dg.template at<7>(k, lane << 2); };
+
+  // exclusive scan of 256 values of shared memory, two per thread
+  auto start_of = [&](uint2 &mine) {
+    mine = *reinterpret_cast<const uint2 *>(s_tot + 2 * t);
+    unsigned before = 0;
+    for (unsigned k = 0; k < 2 * warp; ++k) before += s_tot[32 * k + lane];
+    before = __reduce_add_sync(0xffffffffu, before);
+    unsigned incl = mine.x + mine.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
+      if (lane >= (unsigned)o) incl += v;
     }
-    if (lane == 31) s_scan[warp] = incl;
-    __syncthreads();
-    unsigned before = 0;
-    for (int w = 0; w < warp; ++w) before += s_scan[w];
-    s_run[t] = before + incl - c + prefix[(size_t)t * gridDim.x + blockIdx.x];
-    __syncthreads();
-  }
-  const long long tile_begin = (long long)blockIdx.x * chunk;
-  const long long ntiles = (long long)((n + kRadixTile - 1) / kRadixTile);
-  const long long tile_end = min(ntiles, tile_begin + chunk);
-  const unsigned lt = (1u << lane) - 1u;
-  const int wbase = warp * (32 * kRadixItems);
-  unsigned *wh = s_wh + warp * (kRadixBins + 1);
+    return before + incl - mine.x - mine.y;
+  };
 
-  for (long long tile = tile_begin; tile < tile_end; ++tile) {
-    for (int i = t; i < kRadixWarps * (kRadixBins + 1); i += kRadixThreads) s_wh[i] = 0;
-    __syncthreads();  // also: the previous tile's keys and slots are used up
-    const size_t tile0 = (size_t)tile * kRadixTile;
-    const int count = (int)min((size_t)kRadixTile, n - tile0);
-    // keys of this thread: warp-owned run, 32 consecutive keys per round; a
-    // key's digit (9 bits: 256 = past the end) and its rank among the warp's
-    // keys of that digit (13 bits) share one register
-    T key[kRadixItems];
-    unsigned rd[kRadixItems];
+  // next output slot of this thread's digits 2t and 2t + 1 in this chunk
+  uint2 mine;
+  s_tot[2 * t] = totals[2 * t];
+  s_tot[2 * t + 1] = totals[2 * t + 1];
+  __syncthreads();
+  unsigned run0 = start_of(mine), run1 = run0 + mine.x;
+  run0 += prefix[(size_t)(2 * t) * gridDim.x + blockIdx.x];
+  run1 += prefix[(size_t)(2 * t + 1) * gridDim.x + blockIdx.x];
+
+  const unsigned ntiles = (n + TILE - 1) / TILE;
+  const unsigned tile_begin = (unsigned)(blockIdx.x * chunk);
+  const unsigned tile_end = min(ntiles, tile_begin + (unsigned)chunk);
+  const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+
+  // constants of the rank arithmetic: which byte of an old counter word is
+  // this thread's (as byte_perm selectors), minus S for the bytes of a word
+  // from this thread's on, and the triangular matrix's three kinds of words
+  unsigned sel[4];
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
-      const int j = wbase + r * 32 + lane;
-      if (j < count) key[r] = in[tile0 + j];
+  for (int j = 0; j < 4; ++j) sel[j] = (0x3210u & ~(0xfu << (4 * j))) | ((4u + warp) << (4 * j));
+  const int taken = (int)((((256u - S) & 0xffu) * 0x01010101u) << (8 * warp));
+  const unsigned one = 1u << (8 * warp);
+  const unsigned g = lane >> 2, q = lane & 3u;
+  const unsigned ones = S * 0x01010101u;
+  const unsigned b_lt = q < (g >> 1) ? ones : 0u, b_le = q <= (g >> 1) ? ones : 0u,
+                 b_mid = (g & 1u) ? b_le : b_lt;
+
+  if (tile_begin < tile_end)
+    radix_load_tile<T>(x, in, tile_begin * TILE, min(TILE, n - tile_begin * TILE), vec, pad);
+#pragma unroll
+  for (int i = 0; i < kRadixTileBytes / (kDownThreads * 16); ++i)
+    *reinterpret_cast<uint4 *>(y + (i * kDownThreads + t) * 16) = make_uint4(0, 0, 0, 0);
+
+  for (unsigned tile = tile_begin; tile < tile_end; ++tile) {
+    const unsigned count = min(TILE, n - tile * TILE);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // keys staged in x, counters in y zero
+
+    // count: the keys' ranks among the thread's own keys of their digits
+    T key[K];
+    unsigned rk[K / 4];
+#pragma unroll
+    for (unsigned c = 0; c < 16; ++c) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(x + radix_stage(t, c));
+      memcpy(key + c * (K / 16), &v, 16);
     }
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
-      const int j = wbase + r * 32 + lane;
-      const unsigned d = j < count ? RadixKey<T>::digit(key[r], desc, pass) : (unsigned)kRadixBins;
-      // a full tile has no key past the end: the 9th label bit is always 0
-      const unsigned peers = count == kRadixTile ? radix_peers<kRadixBits>(d) : radix_peers<kRadixBits + 1>(d);
-      const unsigned base = wh[d];
-      rd[r] = ((base + (unsigned)__popc(peers & lt)) << 9) | d;
-      __syncwarp();
-      if (lane == __ffs(peers) - 1) wh[d] = base + (unsigned)__popc(peers);
-      __syncwarp();
+    for (unsigned j = 0; j < K; ++j) {
+      const unsigned old = atomicAdd(reinterpret_cast<unsigned *>(y + counter(key[j])), one);
+      rk[j / 4] = __byte_perm(j % 4 ? rk[j / 4] : 0u, old, sel[j % 4]);
     }
     __syncthreads();
-    for (int d = t; d < kRadixBins; d += kRadixThreads) {
-      // this digit's per-warp counts -> exclusive bases, and the tile count
-      unsigned sum = 0;
+
+    // prefixes of the counter words, warp w: digits 64 w .. 64 w + 63.  Lane
+    // (g, q) holds words 8 q .. 8 q + 7 of rows g and g + 8 (odd rows load
+    // and store their halves the other way round: no bank conflicts).
+    unsigned pk[4][8];  // words 8 q + i: row g in the low half, row g + 8 in the high half
 #pragma unroll
-      for (int w = 0; w < kRadixWarps; ++w) {
-        const unsigned c = s_wh[w * (kRadixBins + 1) + d];
-        s_wh[w * (kRadixBins + 1) + d] = sum;
-        sum += c;
+    for (int m = 0; m < 4; ++m) {
+      unsigned a[2][8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const char *row = y + (64 * warp + 16 * m + 8 * h + g) * 128 + q * 32;
+        const uint4 u = *reinterpret_cast<const uint4 *>(row + 16 * (g & 1u));
+        const uint4 v = *reinterpret_cast<const uint4 *>(row + 16 * (~g & 1u));
+        const bool odd = g & 1u;
+        a[h][0] = odd ? v.x : u.x, a[h][1] = odd ? v.y : u.y, a[h][2] = odd ? v.z : u.z, a[h][3] = odd ? v.w : u.w;
+        a[h][4] = odd ? u.x : v.x, a[h][5] = odd ? u.y : v.y, a[h][6] = odd ? u.z : v.z, a[h][7] = odd ? u.w : v.w;
       }
-      s_tot[d] = sum;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        int d[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+          radix_mma(d, a[0][2 * s], a[1][2 * s], a[0][2 * s + 1], a[1][2 * s + 1],
+                    2 * s <= 2 * j ? b_le : b_lt,
+                    2 * s + 1 <= 2 * j ? b_le : (2 * s + 1 == 2 * j + 1 ? b_mid : b_lt));
+        pk[m][2 * j] = __byte_perm(d[0], d[2], 0x5410);
+        pk[m][2 * j + 1] = __byte_perm(d[1], d[3], 0x5410);
+      }
+      if (q == 3) {  // the last word's prefix is the digit's count
+        s_tot[64 * warp + 16 * m + g] = (pk[m][7] & 0xffffu) / S;
+        s_tot[64 * warp + 16 * m + 8 + g] = (pk[m][7] >> 16) / S;
+      }
     }
     __syncthreads();
-    // first slot of each digit inside the tile: exclusive scan of the counts
-    // (one digit per thread: kRadixThreads == kRadixBins)
     {
-      const unsigned c = s_tot[t];
-      unsigned incl = c;
+      const unsigned start = start_of(mine);
+      *reinterpret_cast<uint2 *>(s_start + 2 * t) = make_uint2(start * S, (start + mine.x) * S);
+      *reinterpret_cast<uint2 *>(s_base + 2 * t) = make_uint2(run0 - start, run1 - (start + mine.x));
+      run0 += mine.x;
+      run1 += mine.y;
+    }
+    __syncwarp();  // a warp's rows are its own threads' digits
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+    for (int m = 0; m < 4; ++m) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const unsigned r = 64 * warp + 16 * m + 8 * h + g, st = s_start[r];
+        unsigned w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = (h ? pk[m][i] >> 16 : pk[m][i] & 0xffffu) + st;
+        const bool odd = g & 1u;
+        char *row = x + r * 128 + q * 32;
+        *reinterpret_cast<uint4 *>(row + 16 * (g & 1u)) =
+            make_uint4(odd ? w[4] : w[0], odd ? w[5] : w[1], odd ? w[6] : w[2], odd ? w[7] : w[3]);
+        *reinterpret_cast<uint4 *>(row + 16 * (~g & 1u)) =
+            make_uint4(odd ? w[0] : w[4], odd ? w[1] : w[5], odd ? w[2] : w[6], odd ? w[3] : w[7]);
       }
-      if (lane == 31) s_scan[warp] = incl;
-      __syncthreads();
-      unsigned before = 0;
-      for (int w = 0; w < warp; ++w) before += s_scan[w];
-      s_lstart[t] = before + incl - c;
     }
     __syncthreads();
-    // reorder the tile by digit in shared memory (stable)
+
+    // each key's place in the sorted tile, in bytes (two 16-bit places per
+    // register); 4- or 8-byte slots swizzled by the place's bits from 10 on,
+    // so that a warp whose keys all have one digit writes different banks
+    constexpr unsigned kSwzShift = S == 4 ? 8 : 7, kSwzMask = S == 4 ? 0x7c : 0x78;
+    unsigned pos[K / 2];
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
-      const unsigned d = rd[r] & 511u;
-      if (d < kRadixBins) {
-        const unsigned pos = s_lstart[d] + s_wh[warp * (kRadixBins + 1) + d] + (rd[r] >> 9);
-        s_keys[pos] = key[r];
-      }
+    for (unsigned j = 0; j < K; ++j) {
+      const unsigned o = counter(key[j]);
+      int p = __dp4a(*reinterpret_cast<const int *>(y + o), taken, *reinterpret_cast<const int *>(x + o));
+      p = __dp4a((int)rk[j / 4], (int)(S << (8 * (j % 4))), p);
+      const unsigned z = (unsigned)p ^ (((unsigned)p >> kSwzShift) & kSwzMask);
+      pos[j / 2] = j % 2 ? pos[j / 2] | (z << 16) : z;
+    }
+    __syncthreads();  // counters and prefixes are used up
+
+    if (tile + 1 < tile_end)
+      radix_load_tile<T>(y, in, (tile + 1) * TILE, min(TILE, n - (tile + 1) * TILE), vec, pad);
+#pragma unroll
+    for (unsigned j = 0; j < K; ++j) {
+      const unsigned z = j % 2 ? pos[j / 2] >> 16 : pos[j / 2] & 0xffffu;
+      *reinterpret_cast<T *>(x + z) = key[j];
     }
     __syncthreads();
+
     // each key to its slot
-    for (int i = t; i < count; i += kRadixThreads) {
-      const T x = s_keys[i];
-      const unsigned d = RadixKey<T>::digit(x, desc, pass);
-      const size_t g = (size_t)s_run[d] + (unsigned)(i - (int)s_lstart[d]);
-      if (g < n) out[g] = x;
+    auto put = [&](unsigned r) {
+      const unsigned i = r * kDownThreads + t;
+      const unsigned z = (i * S) ^ (((r * kDownThreads * S) >> kSwzShift) & kSwzMask);
+      const T k = *reinterpret_cast<const T *>(x + z);
+      const unsigned o = dg.template at<2>(k, 0);
+      const unsigned slot = *reinterpret_cast<const unsigned *>(reinterpret_cast<const char *>(s_base) + o) + i;
+      if (slot < n) out[slot] = k;
+    };
+    if (count == TILE) {
+#pragma unroll 16
+      for (unsigned r = 0; r < K; ++r) put(r);
+    } else {
+      for (unsigned r = 0; r * kDownThreads + t < count; ++r) put(r);
     }
     __syncthreads();
-    s_run[t] += s_tot[t];
+
+    // the sorted tile's buffer takes the next tile's counters
+#pragma unroll
+    for (int i = 0; i < kRadixTileBytes / (kDownThreads * 16); ++i)
+      *reinterpret_cast<uint4 *>(x + (i * kDownThreads + t) * 16) = make_uint4(0, 0, 0, 0);
+    char *const z = x;
+    x = y;
+    y = z;
   }
 }
 
 // Radix sort of keys[0..n) in place (stable, by the key order; descending:
 // the reversed order, still stable).  1 < n < kRadixMaxKeys; scratch:
 // radix_scratch_bytes<T>(n) bytes of device memory, 256-byte aligned.
+// The pad key's digit is 255 in every pass.
+template <class T>
+inline T radix_pad(bool desc) {
+  if constexpr (std::is_floating_point<T>::value) {
+    const unsigned long long u = desc ? ~0ull : ~0ull >> 1;
+    const unsigned v = desc ? ~0u : ~0u >> 1;
+    T x;
+    if constexpr (sizeof(T) == 4) memcpy(&x, &v, 4);
+    else memcpy(&x, &u, 8);
+    return x;
+  } else {
+    return desc ? std::numeric_limits<T>::min() : std::numeric_limits<T>::max();
+  }
+}
+
 template <class T>
 int launch_radix_sort(T *keys, size_t n, bool desc, void *scratch, size_t scratch_bytes, int sm_count,
                       cudaStream_t st) {
-  static_assert(kRadixThreads == kRadixBins, "one digit per thread in the tile scans");
-  constexpr int P = RadixKey<T>::kPasses;
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "4- or 8-byte keys");
+  constexpr int P = (int)sizeof(T) * 8 / kRadixBits;
   if (n <= 1) return B2P_OK;
   if (n >= kRadixMaxKeys || sm_count > 256) return B2P_ERR_UNSUPPORTED;
   const RadixLayout l = radix_layout<T>(n, sm_count);
@@ -323,10 +500,10 @@ int launch_radix_sort(T *keys, size_t n, bool desc, void *scratch, size_t scratc
   const T *src = keys;
   T *dst = buf;
   for (int p = 0; p < P; ++p) {
-    radix_upsweep_kernel<T><<<l.blocks, kRadixThreads, 0, st>>>(src, n, desc, p, l.chunk, counts);
+    radix_upsweep_kernel<T><<<l.blocks, kRadixThreads, 0, st>>>(src, (unsigned)n, desc, p, l.chunk, counts);
     radix_spine_kernel<<<kRadixBins, kRadixSpineThreads, 0, st>>>(counts, l.blocks, totals);
-    radix_downsweep_kernel<T><<<l.blocks, kRadixThreads, smem, st>>>(src, dst, n, desc, p, l.chunk, counts,
-                                                                      totals);
+    radix_downsweep_kernel<T><<<l.blocks, kDownThreads, smem, st>>>(src, dst, (unsigned)n, desc, p, l.chunk, counts,
+                                                                    totals, radix_pad<T>(desc));
     src = dst;
     dst = (dst == buf) ? keys : buf;
   }

@@ -186,3 +186,26 @@ def test_sort_largest_radix_input(dev):
     assert torch.equal(torch.bincount(((x >> 24) & 0xFF).to(torch.int32), minlength=256), h0)
     del x
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("code", [C.I32, C.F32, C.I64, C.F64])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_radix_tile_edges(dev, code, offset):
+    """Around the radix sort's 32 KiB tiles (8192 4-byte or 4096 8-byte keys)
+    and around one tile per resident block, where a block starts to walk
+    several tiles; keys that start 16-byte aligned (staged by cp.async) or one
+    element later; random digits, few distinct keys, and keys already in
+    order (a whole tile in one digit of the upper passes)."""
+    rng = np.random.default_rng(400 + code)
+    tile = 8192 if code in (C.I32, C.F32) else 4096
+    blocks = 3 * torch.cuda.get_device_properties(0).multi_processor_count
+    for n in (8 * tile - 1, 8 * tile, 8 * tile + 1, blocks * tile, blocks * tile + 1, 2 * blocks * tile - 1):
+        for kind in ("random", "dup", "sorted"):
+            x = keys(rng, code, n, kind == "dup")
+            if kind == "sorted":
+                x.sort()
+            desc = bool(n & 1)
+            t = torch.empty(n + offset, dtype=dev_t(x[:1]).dtype, device="cuda")[offset:]
+            t.copy_(dev_t(x))
+            C.sort_(t, descending=desc)
+            assert same_bits(t.cpu().numpy(), O.sort(x, desc)), (n, kind)
