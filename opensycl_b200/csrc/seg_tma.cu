@@ -60,13 +60,16 @@ constexpr int kSegNeedCarry = 2;  // some output of the tile needs the carry
 constexpr unsigned long long kSegTexclF = 1ull << 63;  // the thread's exclusive prefix has a head
 
 // Boundary i of the tile, relative to the tile's first element (the staged
-// record, or global memory when the tile has more than a record holds).
+// record, or global memory when the tile has more than a record holds).  A
+// record holds its boundaries shifted left by 8: records lie in the scratch
+// body, where a later launch of another shape keeps status words, and a word
+// whose flag byte is zero is never taken for a published one.
 struct SegBounds {
   const int *s;
   const long long *g;
   long long t0;
   int m;
-  __device__ __forceinline__ long long at(int i) const { return s ? (long long)s[i] : g[i] - t0; }
+  __device__ __forceinline__ long long at(int i) const { return s ? (long long)(s[i] >> 8) : g[i] - t0; }
   // first i with at(i) >= v
   __device__ __forceinline__ int lower(long long v) const {
     int lo = 0, hi = m;
@@ -861,7 +864,7 @@ void segmented_tile_records(const int64_t *offs, int64_t nseg, size_t n, int blo
     r[0] = (int)k;
     r[1] = (int)m;
     for (int i = 0; i < kSegRecCap; ++i)
-      r[2 + i] = i < m ? (int)std::min<int64_t>(offs[k + i] - t0, (int64_t)tile + 1) : 0;
+      r[2 + i] = i < m ? (int)std::min<int64_t>(offs[k + i] - t0, (int64_t)tile + 1) << 8 : 0;
   }
 }
 

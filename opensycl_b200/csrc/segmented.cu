@@ -28,9 +28,13 @@ namespace b2p {
 
 constexpr int kMaxSegsPerPiece = 64;
 
+// Pieces lie in the scratch body, where a later launch of another shape keeps
+// status words: the byte that is a status word's flags (the low byte of every
+// second 8 bytes) is zero in a piece, so that it is never taken for a
+// published word.
 struct __align__(16) Piece {
   long long elem_begin;  // first element
-  int elem_count;        // elements in the piece
+  int elem_count_8;      // elements in the piece, shifted left by 8
   int seg_begin;         // first segment
   int seg_count;         // segments (whole ones, or 1 for a long segment)
   int flags;             // kPieceFirst | kPieceLast | kPieceMulti
@@ -84,7 +88,7 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
     const long long item = (long long)s_item;
     if (item >= p.npieces) break;
     const Piece pc = p.pieces[item];
-    const int count = min(pc.elem_count, tile_elems);
+    const int count = min(pc.elem_count_8 >> 8, tile_elems);
     const bool multi = (pc.flags & kPieceMulti) != 0;
     const int nsegs = min(pc.seg_count, kMaxSegsPerPiece);
     // elements (coalesced scalar loads: pieces start anywhere) and, for a
@@ -221,7 +225,7 @@ std::vector<Piece> build_pieces(const int64_t *offs, int64_t nseg, int cap) {
       for (int64_t k = 0; k < np; ++k) {
         Piece pc{};
         pc.elem_begin = offs[s] + k * cap;
-        pc.elem_count = (int)std::min<int64_t>(cap, len - k * cap);
+        pc.elem_count_8 = (int)std::min<int64_t>(cap, len - k * cap) << 8;
         pc.seg_begin = (int)s;
         pc.seg_count = 1;
         pc.flags = (k == 0 ? kPieceFirst : 0) | (k == np - 1 ? kPieceLast : 0);
@@ -241,7 +245,7 @@ std::vector<Piece> build_pieces(const int64_t *offs, int64_t nseg, int cap) {
       total += l;
       ++e;
     }
-    pc.elem_count = (int)total;
+    pc.elem_count_8 = (int)total << 8;
     pc.seg_count = (int)(e - s);
     v.push_back(pc);
     s = e;

@@ -113,3 +113,25 @@ def test_segmented_plan_graph(dev):
         assert np.array_equal(out.cpu().numpy(), ref)
     assert 0 <= L.b2p_plan_config(plan) < 48
     L.b2p_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("flat", [18, 22, 23])
+def test_segmented_kernels_share_scratch_at_every_epoch(dev, flat):
+    """The pipelined kernel's boundary records (a tile without a boundary
+    inside holds tile + 1 = 0x801, 0x1001 or 0x2001) and the piece kernel's
+    pieces stay in the scratch body; a look-back of the other kernel over the
+    same bytes must not take one for a status word of its launch, whatever
+    the launch's epoch (those values once read as "aggregate of epoch 8, 16
+    or 32")."""
+    rng = np.random.default_rng(flat)
+    lens = rng.integers(20000, 40000, 60)
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    x = values(rng, C.I32, int(offs[-1]))
+    xd, od = torch.from_numpy(x).cuda(), torch.from_numpy(offs).cuda()
+    ref = O.segmented_reduce(C.I32, C.SUM, x, offs)
+    C.Scratch.release()
+    C.Scratch.get(C.lib().b2p_scratch_bytes(C.PRIM_SEG_REDUCE, C.I32, x.size, 60, C.AUTO) + 256)
+    assert np.array_equal(C.segmented_reduce(xd, od, "sum", config=0).cpu().numpy(), ref)  # epoch 0
+    for epoch in range(1, 35, 2):
+        assert np.array_equal(C.segmented_reduce(xd, od, "sum", config=flat).cpu().numpy(), ref), epoch
+        assert np.array_equal(C.segmented_reduce(xd, od, "sum", config=0).cpu().numpy(), ref), epoch + 1
