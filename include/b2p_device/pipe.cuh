@@ -86,7 +86,7 @@ struct TmaParams {
   // ints: the index kb of the first offset at or after the tile's first
   // element, the count m of offsets from kb up to and including the first
   // one at or after the tile's end, and those m offsets relative to the
-  // tile's first element when they fit)
+  // tile's first element, shifted left by 8, when they fit)
   const long long *offsets;
   long long nseg;
   const int *seg_rec;

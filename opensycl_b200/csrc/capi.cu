@@ -363,25 +363,22 @@ static int segmented_reduce_entry(int dtype, int op, const void *in, const int64
   if ((rc = check_ptr(in, dtype_size(dtype))) || (rc = check_ptr(out, acc_size(dtype))) ||
       (rc = check_ptr(offsets, 8)))
     return rc;
-  // total element count is needed on the host: read offsets[nseg]
-  int64_t total = 0;
-  cudaError_t e = cudaMemcpyAsync(&total, offsets + nseg, sizeof(int64_t), cudaMemcpyDefault,
-                                  (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
-  if (e != cudaSuccess) return cuda_status(e);
+  // the total element count is needed on the host
+  SegOffsets o;
+  if ((rc = check_extent(offsets, 8 * ((size_t)nseg + 1)))) return rc;
+  if ((rc = read_offsets(offsets, nseg, scratch, scratch_bytes, o, (cudaStream_t)stream))) return rc;
+  const int64_t total = o.total;
   if (total < 0) return B2P_ERR_INVALID_ARG;
   cs.set_size((size_t)total, (double)total * dtype_size(dtype) + (double)nseg * (acc_size(dtype) + 8));
   if ((rc = check_extent(in, (size_t)total * dtype_size(dtype))) ||
       (rc = check_extent(out, (size_t)nseg * acc_size(dtype))) ||
-      (rc = check_extent(offsets, 8 * ((size_t)nseg + 1))) ||
       (rc = check_offsets(offsets, nseg, (size_t)total, (cudaStream_t)stream)))
     return rc;
   if (!scratch) return B2P_ERR_SCRATCH;
   config = resolve(B2P_PRIM_SEG_REDUCE, dtype, (size_t)total, nseg, config);
   if (!config_valid(B2P_PRIM_SEG_REDUCE, dtype, config)) return B2P_ERR_INVALID_ARG;
-  return launch_segmented(B2P_PRIM_SEG_REDUCE, dtype, op, 1, in, out, offsets, nseg,
-                          (size_t)total, init, scratch, scratch_bytes, config,
-                          (cudaStream_t)stream);
+  return launch_segmented(B2P_PRIM_SEG_REDUCE, dtype, op, 1, in, out, offsets, nseg, o, init, scratch,
+                          scratch_bytes, config, (cudaStream_t)stream);
 }
 
 int b2p_segmented_reduce(int dtype, int op, const void *in, const int64_t *offsets, int64_t nseg,
@@ -402,25 +399,22 @@ static int segmented_scan_entry(int dtype, int op, int inclusive, const void *in
   if ((rc = check_ptr(in, dtype_size(dtype))) || (rc = check_ptr(out, acc_size(dtype))) ||
       (rc = check_ptr(offsets, 8)))
     return rc;
-  int64_t total = 0;
-  cudaError_t e = cudaMemcpyAsync(&total, offsets + nseg, sizeof(int64_t), cudaMemcpyDefault,
-                                  (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
-  if (e != cudaSuccess) return cuda_status(e);
+  SegOffsets o;
+  if ((rc = check_extent(offsets, 8 * ((size_t)nseg + 1)))) return rc;
+  if ((rc = read_offsets(offsets, nseg, scratch, scratch_bytes, o, (cudaStream_t)stream))) return rc;
+  const int64_t total = o.total;
   if (total < 0) return B2P_ERR_INVALID_ARG;
   if (total == 0) return B2P_OK;
   cs.set_size((size_t)total, (double)total * (dtype_size(dtype) + acc_size(dtype)) + 8.0 * nseg);
   if ((rc = check_extent(in, (size_t)total * dtype_size(dtype))) ||
       (rc = check_extent(out, (size_t)total * acc_size(dtype))) ||
-      (rc = check_extent(offsets, 8 * ((size_t)nseg + 1))) ||
       (rc = check_offsets(offsets, nseg, (size_t)total, (cudaStream_t)stream)))
     return rc;
   if (!scratch) return B2P_ERR_SCRATCH;
   config = resolve(B2P_PRIM_SEG_SCAN, dtype, (size_t)total, nseg, config);
   if (!config_valid(B2P_PRIM_SEG_SCAN, dtype, config)) return B2P_ERR_INVALID_ARG;
-  return launch_segmented(B2P_PRIM_SEG_SCAN, dtype, op, inclusive, in, out, offsets, nseg,
-                          (size_t)total, init, scratch, scratch_bytes, config,
-                          (cudaStream_t)stream);
+  return launch_segmented(B2P_PRIM_SEG_SCAN, dtype, op, inclusive, in, out, offsets, nseg, o, init, scratch,
+                          scratch_bytes, config, (cudaStream_t)stream);
 }
 
 int b2p_segmented_scan(int dtype, int op, int inclusive, const void *in, void *out,

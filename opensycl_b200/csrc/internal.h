@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "../../include/b2p.h"
 
@@ -54,6 +55,8 @@ void note_config(int config);
 // B2P_CHECKED: extents of pointer arguments and segment offsets are checked.
 bool checked_mode();
 int check_extent(const void *p, size_t bytes);
+// Whether the bytes are known to lie inside one device allocation (in any mode).
+bool inside_allocation(const void *p, size_t bytes);
 int check_offsets(const int64_t *offsets, int64_t nseg, size_t total, cudaStream_t st);
 // B2P_SELECTOR: 0 = installed selector table, else heuristic; 1 = heuristic.
 int selector_mode();
@@ -131,19 +134,30 @@ int launch_histogram_u8(const uint8_t *keys, size_t n, uint32_t *bins, int nbins
 
 // Segmented reduce / scan (one persistent launch).
 size_t segmented_scratch_bytes(int dtype, size_t n, int64_t nseg, int config);
+// The offsets of a segmented call as the host needs them: the total, whether
+// they can be used (non-negative, non-decreasing), and, for a short array, the
+// offsets themselves.
+struct SegOffsets {
+  int64_t first = 0, total = 0;
+  bool checked = false, valid = false;  // valid: once checked
+  std::vector<int64_t> host;  // empty: not copied
+};
+int read_offsets(const int64_t *offsets, int64_t nseg, void *scratch, size_t scratch_bytes, SegOffsets &o,
+                 cudaStream_t s);
 int launch_segmented(int prim, int dtype, int op, int inclusive, const void *in, void *out,
-                     const int64_t *offsets, int64_t nseg, size_t total, const void *init,
+                     const int64_t *offsets, int64_t nseg, SegOffsets &o, const void *init,
                      void *scratch, size_t scratch_bytes, int config, cudaStream_t s);
 bool segmented_config_valid(int dtype, int config);
 // The pipelined segmented kernel (flat segmented scan on the TMA pipeline):
 // whether it has the (dtype, op, block, items) shape, the scratch it needs
 // (prefix, one status word per tile, then one 64-int record per tile), the
-// host computation of the records, and the launch.  The records must
-// already be in scratch; returns B2P_ERR_UNSUPPORTED, having launched
-// nothing, when the call does not fit.
+// kernel that writes the records into scratch, and the launch.  The records
+// must be written before it on the stream; returns B2P_ERR_UNSUPPORTED, having
+// launched nothing, when the call does not fit.
 bool segmented_tma_shape(int dtype, int op, int block, int items);
 size_t segmented_tma_scratch(size_t n, int block, int items);
-void segmented_tile_records(const int64_t *offs, int64_t nseg, size_t n, int block, int items, int *rec);
+int launch_segmented_records(const int64_t *offsets, int64_t nseg, size_t n, int block, int items, void *scratch,
+                             cudaStream_t s);
 int launch_segmented_tma(int prim, int dtype, int op, int inclusive, const void *in, void *out,
                          const int64_t *offsets, int64_t nseg, size_t n, const void *init, void *scratch,
                          int block, int items, cudaStream_t s);

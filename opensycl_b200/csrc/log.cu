@@ -138,6 +138,15 @@ int check_extent(const void *p, size_t bytes) {
   return B2P_OK;
 }
 
+bool inside_allocation(const void *p, size_t bytes) {
+  AddressRangeFn fn = address_range_fn();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (!fn || fn(&base, &size, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+  const uintptr_t a = (uintptr_t)p, b0 = (uintptr_t)base;
+  return a >= b0 && a - b0 <= size && bytes <= size - (a - b0);
+}
+
 int check_offsets(const int64_t *offsets, int64_t nseg, size_t total, cudaStream_t st) {
   if (!checked_mode()) return B2P_OK;
   std::vector<int64_t> h((size_t)nseg + 1);

@@ -404,60 +404,135 @@ int seg_launch_with_pieces(int prim, int dtype, int op, int inclusive, const voi
 // Whether a call runs the pipelined flat kernel (seg_tma.cu): grid mode 1
 // with a shape it has, SUM, offsets starting at 0, 16-byte aligned input
 // (and output for a scan), at least one tile of elements.
-bool seg_tma_fits(int prim, int dtype, int op, int config, const void *in, const void *out, const int64_t *h,
+bool seg_tma_fits(int prim, int dtype, int op, int config, const void *in, const void *out, int64_t first,
                   int64_t nseg, size_t total) {
   const LaunchConfig lc = describe_config(config);
   if (lc.grid_mode != 1 || !segmented_tma_shape(dtype, op, lc.block, lc.items)) return false;
-  if (h[0] != 0 || nseg >= (1ll << 31) - 2 || total < (size_t)lc.block * lc.items) return false;
+  if (first != 0 || nseg >= (1ll << 31) - 2 || total < (size_t)lc.block * lc.items) return false;
   if (reinterpret_cast<uintptr_t>(in) & 15) return false;
   if (prim == B2P_PRIM_SEG_SCAN && (reinterpret_cast<uintptr_t>(out) & 15)) return false;
   return true;
 }
 
-// The per-tile records of the pipelined kernel, copied into scratch after
-// its status words (synchronous: the records are a host temporary).
-int seg_tma_prepare(const int64_t *h, int64_t nseg, size_t total, int config, void *scratch, size_t scratch_bytes,
-                    cudaStream_t st) {
+// The per-tile records of the pipelined kernel, written into scratch after its
+// status words.
+int seg_tma_prepare(const int64_t *offsets, int64_t nseg, size_t total, int config, void *scratch,
+                    size_t scratch_bytes, cudaStream_t st) {
   const LaunchConfig lc = describe_config(config);
   if (scratch_bytes < segmented_tma_scratch(total, lc.block, lc.items)) return B2P_ERR_SCRATCH;
-  const size_t tile = (size_t)lc.block * lc.items, ntiles = (total + tile - 1) / tile;
-  std::vector<int> tk(ntiles * 64);
-  segmented_tile_records(h, nseg, total, lc.block, lc.items, tk.data());
-  char *dst = reinterpret_cast<char *>(scratch) + kScratchPrefix + ntiles * sizeof(StatusWord);
-  cudaError_t e = cudaMemcpyAsync(dst, tk.data(), tk.size() * sizeof(int), cudaMemcpyHostToDevice, st);
+  return launch_segmented_records(offsets, nseg, total, lc.block, lc.items, scratch, st);
+}
+
+namespace {
+
+// What the host has to know of long offsets: the first, the last, and whether
+// one is below the one before it.
+struct SegCheck {
+  long long first, last;
+  unsigned decreasing, pad;
+};
+// in the scratch header, after the control block
+constexpr size_t kSegCheckAt = 128;
+static_assert(kSegCheckAt >= sizeof(ScratchHeader) && kSegCheckAt + sizeof(SegCheck) <= kHeaderBytes, "header room");
+constexpr int kSegCheckThreads = 1024;
+
+__global__ void __launch_bounds__(kSegCheckThreads) seg_check_kernel(const long long *offs, long long nseg,
+                                                                     SegCheck *c) {
+  int bad = 0;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += step)
+    bad |= offs[i + 1] < offs[i];
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    if (gridDim.x == 1) c->decreasing = bad;
+    else if (bad) atomicOr(&c->decreasing, 1u);
+    if (blockIdx.x == 0) {
+      c->first = offs[0];
+      c->last = offs[nseg];
+    }
+  }
+}
+
+// Up to this many segments the offsets themselves are copied to the host (one
+// copy then serves the checks and the piece map); longer arrays are checked on
+// the device and only the result comes back.  (The copy refuses an array that
+// runs past its allocation; so does the device's path, which only takes arrays
+// known to lie inside one.)  Around the limit both routes take the same time
+// (2^24 floats: 54 us a call with 1,024 and with 1,100 segments); beyond it
+// the copy and the host's check grow with the array, the kernel's 3 us hardly.
+constexpr int64_t kSegHostOffsets = 1024;
+
+// Copies all offsets to the host and checks them.
+int copy_offsets(const int64_t *offsets, int64_t nseg, SegOffsets &o, cudaStream_t st) {
+  o.host.resize((size_t)nseg + 1);
+  cudaError_t e = cudaMemcpyAsync(o.host.data(), offsets, o.host.size() * sizeof(int64_t), cudaMemcpyDefault, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  return cuda_status(e);
+  if (e != cudaSuccess) return cuda_status(e);
+  o.first = o.host[0];
+  o.total = o.host[(size_t)nseg];
+  o.valid = o.first >= 0;
+  for (int64_t s = 0; s < nseg && o.valid; ++s) o.valid = o.host[(size_t)s + 1] >= o.host[(size_t)s];
+  o.checked = true;
+  return B2P_OK;
+}
+
+}  // namespace
+
+int read_offsets(const int64_t *offsets, int64_t nseg, void *scratch, size_t scratch_bytes, SegOffsets &o,
+                 cudaStream_t st) {
+  if (nseg <= kSegHostOffsets) return copy_offsets(offsets, nseg, o, st);
+  const bool on_device = scratch && scratch_bytes >= kHeaderBytes && check_pointer(scratch, 256) == B2P_OK &&
+                         inside_allocation(offsets, ((size_t)nseg + 1) * sizeof(int64_t));
+  if (!on_device) {  // the total alone; launch_segmented copies the rest
+    cudaError_t e = cudaMemcpyAsync(&o.total, offsets + nseg, sizeof(int64_t), cudaMemcpyDefault, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    return cuda_status(e);
+  }
+  SegCheck *dc = reinterpret_cast<SegCheck *>(reinterpret_cast<char *>(scratch) + kSegCheckAt), c;
+  const int grid = (int)std::min<int64_t>((nseg + 16 * kSegCheckThreads - 1) / (16 * kSegCheckThreads),
+                                          device_info().sm_count);
+  cudaError_t e = grid > 1 ? cudaMemsetAsync(dc, 0, sizeof(SegCheck), st) : cudaSuccess;
+  if (e != cudaSuccess) return cuda_status(e);
+  seg_check_kernel<<<grid, kSegCheckThreads, 0, st>>>(reinterpret_cast<const long long *>(offsets), nseg, dc);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&c, dc, sizeof(c), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_status(e);
+  o.first = c.first;
+  o.total = c.last;
+  o.valid = c.first >= 0 && !c.decreasing;
+  o.checked = true;
+  return B2P_OK;
 }
 
 int launch_segmented(int prim, int dtype, int op, int inclusive, const void *in, void *out,
-                     const int64_t *offsets, int64_t nseg, size_t total, const void *init,
+                     const int64_t *offsets, int64_t nseg, SegOffsets &o, const void *init,
                      void *scratch, size_t scratch_bytes, int config, cudaStream_t st) {
   if (!seg_tile_ok(dtype, config)) return B2P_ERR_INVALID_ARG;
   if (reinterpret_cast<uintptr_t>(scratch) & 255) return B2P_ERR_SCRATCH;
+  const size_t total = (size_t)o.total;
+  int rc = o.checked ? B2P_OK : copy_offsets(offsets, nseg, o, st);
+  if (rc) return rc;
+  if (!o.valid || (size_t)o.total != total) return B2P_ERR_INVALID_ARG;
   LaunchConfig lc = describe_config(config);
   const int cap = lc.block * lc.items;
-  // the piece map is built on the host from the offsets (one copy back)
-  std::vector<int64_t> h((size_t)nseg + 1);
-  cudaError_t e = cudaMemcpyAsync(h.data(), offsets, h.size() * sizeof(int64_t), cudaMemcpyDefault, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return cuda_status(e);
-  for (int64_t s = 0; s < nseg; ++s)
-    if (h[(size_t)s + 1] < h[(size_t)s] || h[0] < 0) return B2P_ERR_INVALID_ARG;
-  if ((size_t)h[(size_t)nseg] != total) return B2P_ERR_INVALID_ARG;
-  if (seg_tma_fits(prim, dtype, op, config, in, out, h.data(), nseg, total)) {
-    int rc = seg_tma_prepare(h.data(), nseg, total, config, scratch, scratch_bytes, st);
+  if (seg_tma_fits(prim, dtype, op, config, in, out, o.first, nseg, total)) {
+    rc = seg_tma_prepare(offsets, nseg, total, config, scratch, scratch_bytes, st);
     if (rc) return rc;
     rc = launch_segmented_tma(prim, dtype, op, inclusive, in, out, offsets, nseg, total, init, scratch, lc.block,
                               lc.items, st);
     if (rc != B2P_ERR_UNSUPPORTED) return rc;
   }
-  std::vector<Piece> pieces = build_pieces(h.data(), nseg, cap);
+  // the piece map is built on the host from the offsets
+  if (o.host.empty() && (rc = copy_offsets(offsets, nseg, o, st))) return rc;
+  if (!o.valid || (size_t)o.total != total) return B2P_ERR_INVALID_ARG;
+  std::vector<Piece> pieces = build_pieces(o.host.data(), nseg, cap);
   const size_t np = pieces.size();
   const size_t need = kScratchPrefix + np * (sizeof(StatusWord) + sizeof(Piece));
   if (scratch_bytes < need) return B2P_ERR_SCRATCH;
   Piece *dp = reinterpret_cast<Piece *>(reinterpret_cast<char *>(scratch) + kScratchPrefix +
                                         np * sizeof(StatusWord));
-  e = cudaMemcpyAsync(dp, pieces.data(), np * sizeof(Piece), cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemcpyAsync(dp, pieces.data(), np * sizeof(Piece), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // `pieces` is a host temporary
   if (e != cudaSuccess) return cuda_status(e);
   return seg_launch_with_pieces(prim, dtype, op, inclusive, in, out, offsets, nseg, init, dp,
@@ -508,7 +583,7 @@ int b2p_plan_segmented(b2p_plan *plan, int prim, int dtype, int op, const void *
   }
   if (!seg_tile_ok(dtype, config)) return B2P_ERR_INVALID_ARG;
   LaunchConfig lc = describe_config(config);
-  const bool flat = seg_tma_fits(prim, dtype, op, config, in, out, h.data(), nseg, total_elems);
+  const bool flat = seg_tma_fits(prim, dtype, op, config, in, out, h[0], nseg, total_elems);
   std::vector<Piece> pieces = build_pieces(h.data(), nseg, lc.block * lc.items);
   const size_t np = pieces.size();
   b2p_plan_s *pl = new b2p_plan_s();
@@ -543,7 +618,8 @@ int b2p_plan_segmented(b2p_plan *plan, int prim, int dtype, int op, const void *
       break;
     }
     if (use_flat) {
-      rc = seg_tma_prepare(h.data(), nseg, total_elems, config, pl->scratch, pl->scratch_bytes, st);
+      rc = seg_tma_prepare(offsets, nseg, total_elems, config, pl->scratch, pl->scratch_bytes, st);
+      if (rc == B2P_OK) rc = cuda_status(cudaStreamSynchronize(st));
       if (rc) break;
     }
     // capture the single launch into a graph

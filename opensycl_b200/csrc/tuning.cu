@@ -169,8 +169,6 @@ int tune_shape(int prim, int dtype, int op, size_t n, int64_t nseg, double cv, i
     }
     case B2P_PRIM_COPY_IF: return b2p_copy_if(dtype == B2P_BF16 ? B2P_U32 : dtype, in, out, n, 7, B2P_CMP_LT, 3, count, scratch, sbytes, c, (b2p_stream)st);
     case B2P_PRIM_HISTOGRAM: return b2p_histogram_u8((const uint8_t *)in, n, (uint32_t *)out, 256, c, (b2p_stream)st);
-    case B2P_PRIM_SEG_REDUCE: return launch_segmented(prim, dtype, op, 1, in, out, offs, ns, n, nullptr, scratch, sbytes, c, st);
-    case B2P_PRIM_SEG_SCAN: return launch_segmented(prim, dtype, op, 1, in, out, offs, ns, n, nullptr, scratch, sbytes, c, st);
     default: return B2P_ERR_INVALID_ARG;
     }
   };

@@ -135,3 +135,35 @@ def test_segmented_kernels_share_scratch_at_every_epoch(dev, flat):
     for epoch in range(1, 35, 2):
         assert np.array_equal(C.segmented_reduce(xd, od, "sum", config=flat).cpu().numpy(), ref), epoch
         assert np.array_equal(C.segmented_reduce(xd, od, "sum", config=0).cpu().numpy(), ref), epoch + 1
+
+
+@pytest.mark.parametrize("nseg", [1024, 1025, 16 * 1024 + 1, 40000])
+def test_segmented_offsets_checked_on_device(dev, nseg):
+    """Offset arrays on both sides of the limits of the device-side check (one
+    block up to 16,384 segments) and of a tile's boundary record (62): many
+    empty segments at one place and at the end, hundreds of boundaries in one
+    tile, and one long segment over many tiles.  A decreasing pair anywhere,
+    or a negative first offset, is refused and leaves the output alone."""
+    rng = np.random.default_rng(nseg)
+    lens = rng.integers(0, 30, nseg)
+    lens[nseg // 3:nseg // 3 + 200] = 0
+    lens[nseg // 2] = 300000
+    lens[-5:] = 0
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    x = values(rng, C.I64, int(offs[-1]))
+    xd, od = torch.from_numpy(x).cuda(), torch.from_numpy(offs).cuda()
+    got = C.segmented_reduce(xd, od, "sum").cpu().numpy()
+    assert np.array_equal(got, O.segmented_reduce(C.I64, C.SUM, x, offs))
+    got = C.segmented_scan(xd, od, False, "sum", 5).cpu().numpy()
+    assert np.array_equal(got, O.segmented_scan(C.I64, C.SUM, False, x, offs, 5))
+    for at in (1, nseg // 2 + 1, nseg - 1):
+        bad = offs.copy()
+        bad[at] = bad[at + 1] + 1
+        out = torch.full((nseg,), 7, dtype=torch.int64, device="cuda")
+        with pytest.raises(C.B2PError) as e:
+            C.segmented_reduce(xd, torch.from_numpy(bad).cuda(), "sum", out=out)
+        assert e.value.status == C.ERR_INVALID_ARG and bool((out == 7).all())
+    bad = offs.copy()
+    bad[0] = -1
+    with pytest.raises(C.B2PError):
+        C.segmented_reduce(xd, torch.from_numpy(bad).cuda(), "sum")
