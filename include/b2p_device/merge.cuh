@@ -12,7 +12,8 @@
 //          block stages its tile's two input ranges in shared memory and
 //          every thread merges its ITEMS outputs after its own merge-path
 //          search in shared memory; outputs leave in coalesced rows.
-//          Reads each input once, writes each output once.
+//          Reads each input once, writes each output once.  Standard keys
+//          have a kernel of their own (merge_keys_kernel).
 //   sort   a merge sort: blocks sort tiles in shared memory (a stable
 //          odd-even sort of each thread's ITEMS keys in registers, then
 //          log2(threads) rounds of merge-path merges of runs in shared
@@ -28,6 +29,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <limits>
 
 namespace b2p {
 
@@ -88,6 +90,32 @@ __device__ __forceinline__ long long merge_path_warp(IdxA a, long long na, IdxB 
     const long long new_hi = j == 32 ? hi : lo + span * (j + 1) / 33;
     lo = new_lo;
     hi = new_hi;
+  }
+  return lo;
+}
+
+// merge_path() by groups of G lanes, each group with its own diagonal and
+// range [lo, hi] (which must hold the answer): a range of `span` shrinks to
+// about span / (G + 1) per round.  All 32 lanes call it; every lane of a group
+// returns the group's value.
+template <int G, class Int, class Comp, class IdxA, class IdxB>
+__device__ __forceinline__ Int merge_path_groups(IdxA a, IdxB b, Int lo, Int hi, Int diag, const Comp &comp) {
+  const int lane = threadIdx.x & 31, gl = lane % G;
+  constexpr unsigned kMask = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+  while (__any_sync(0xffffffffu, lo < hi)) {
+    const Int span = hi - lo;
+    const bool few = span <= G;
+    const Int pk = few ? lo + gl : lo + span * (gl + 1) / (G + 1);
+    const bool p = pk < hi && comp(b(diag - 1 - pk), a(pk));
+    const unsigned m = (__ballot_sync(0xffffffffu, p) >> (lane - gl)) & kMask;
+    const int j = m ? __ffs(m) - 1 : G;
+    const Int at = lo;
+    if (few) {
+      lo = hi = m ? at + j : hi;
+    } else {
+      if (j > 0) lo = at + span * j / (G + 1) + 1;
+      if (j < G) hi = at + span * (j + 1) / (G + 1);
+    }
   }
   return lo;
 }
@@ -311,6 +339,250 @@ __global__ void __launch_bounds__(kMergeThreads) block_sort_kernel(T *keys, long
   for (int k = threadIdx.x; k < cnt; k += kMergeThreads) keys[t0 + k] = src[spad(k)];
 }
 
+// ------------------------------------------------- merge of standard keys
+//
+// The same merge for int, float and 64-bit keys under < or >, where a key is
+// its own order.  The keys of a thread's ITEMS outputs are read as an ascending
+// run of a followed by a descending run of b (begun one key late, at a key that
+// is no earlier than any of them), which the log2(ITEMS + 1) rounds of a
+// bitonic merge sort in registers (a min and a max per two keys and round),
+// instead of a serial merge whose every output takes about 16 instructions and
+// waits for a shared load.  ITEMS is odd: the threads' searches start, and
+// their outputs lie, in different banks.  Keys that compare equal have the same bits, so
+// their order cannot be seen; a thread that meets an exception, a -0.0 (equal
+// to +0.0) or a NaN (unordered), merges serially, and so does one whose
+// outputs run past the end.
+//
+// 133 M floats: 229 us, 4.65 TB/s (the serial merge's kernel took 283 us); 2^28
+// int32: 455 us (559).  Bound by latency between its barriers at 25 warps per
+// SM, with the shared-memory pipe 63 % and the ALU pipe 49 % busy; the random
+// banks of the windows and searches are two thirds of the wavefronts.
+template <class T>
+struct MergeNet {
+  static constexpr int kItems = sizeof(T) == 4 ? 31 : 15, kThreads = 160, kBlocksPerSm = 5;
+  static constexpr int kTile = kItems * kThreads;  // no smaller than merge_tile<T>(): no more tile starts
+  // a staged tile: both sides from and to 16-byte boundaries, a key after b
+  static constexpr int kSlots = kTile + 5 * 16 / (int)sizeof(T);
+};
+
+template <class T, bool DESC>
+struct KeyOrder {
+  __device__ __forceinline__ bool operator()(const T &x, const T &y) const { return DESC ? y < x : x < y; }
+  __device__ __forceinline__ static T first(T x, T y) {
+    if constexpr (std::is_same<T, float>::value) return DESC ? fmaxf(x, y) : fminf(x, y);
+    else return DESC ? (x < y ? y : x) : (y < x ? y : x);
+  }
+  __device__ __forceinline__ static T second(T x, T y) {
+    if constexpr (std::is_same<T, float>::value) return DESC ? fminf(x, y) : fmaxf(x, y);
+    else return DESC ? (x < y ? x : y) : (y < x ? x : y);
+  }
+  // a key that none goes after
+  __device__ __forceinline__ static T last_key() {
+    using L = std::numeric_limits<T>;
+    if constexpr (std::is_floating_point<T>::value) return DESC ? -L::infinity() : L::infinity();
+    else return DESC ? L::min() : L::max();
+  }
+  // a key whose order against an equal or any other key is not in its bits
+  __device__ __forceinline__ static bool special(T x) {
+    if constexpr (std::is_same<T, float>::value) {
+      const unsigned u = __float_as_uint(x);
+      return u == 0x80000000u || (u << 1) > 0xff000000u;
+    } else if constexpr (std::is_same<T, double>::value) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+      return u == 0x8000000000000000ull || (u << 1) > 0xffe0000000000000ull;
+    } else {
+      return false;
+    }
+  }
+};
+
+// splits[t] = keys of a before output t * kTile.  A warp takes TILES tiles: the
+// merge path at both ends of their outputs (16 lanes each), then each tile's
+// start between them (32 / TILES lanes each).  TILES = 1: one 32-lane search
+// per tile, the fewest rounds of latency (2.8 us for 167 tiles of two 64-bit
+// sides, against 6.7 us for eight tiles a warp), but 345 scattered sectors a
+// tile: 85 us for 133 M floats, where 32 tiles a warp take 27 us.
+template <class T, bool DESC, int TILES>
+__global__ void __launch_bounds__(128) merge_keys_partition_kernel(const T *a, long long na, const T *b, long long nb,
+                                                                   long long ntiles, long long *splits) {
+  constexpr long long kTile = MergeNet<T>::kTile;
+  const KeyOrder<T, DESC> comp;
+  const int lane = threadIdx.x & 31;
+  const long long t0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * TILES;
+  if (t0 >= ntiles) return;  // whole warps leave together
+  auto ga = [&](long long i) { return a[i]; };
+  auto gb = [&](long long i) { return b[i]; };
+  const long long d0 = t0 * kTile;
+  if constexpr (TILES == 1) {
+    const long long i = merge_path_warp<T>(ga, na, gb, nb, d0, comp);
+    if (lane == 0) splits[t0] = i;
+  } else {
+    constexpr int G = 32 / TILES;
+    const long long d1 = min(d0 + TILES * kTile, na + nb);
+    long long d = lane < 16 ? d0 : d1;
+    const long long e = merge_path_groups<16, long long>(ga, gb, d > nb ? d - nb : 0, min(d, na), d, comp);
+    const long long i0 = __shfl_sync(0xffffffffu, e, 0), i1 = __shfl_sync(0xffffffffu, e, 16);
+    const long long t = t0 + lane / G;
+    d = min(t * kTile, d1);
+    // outputs [d0, d) take at least d - (keys of b up to d1), and no more than
+    // d - (keys of b up to d0), keys of a
+    const long long i =
+        merge_path_groups<G, long long>(ga, gb, max(i0, d - (d1 - i1)), min(i1, d - (d0 - i0)), d, comp);
+    if (lane % G == 0 && t < ntiles) splits[t] = i;
+  }
+}
+
+// One side of a tile, keys [0, count) from src, into the 16-byte chunks of
+// `slots` from chunk c0 on, by cp.async: chunks as they lie in memory, so the
+// first key is at slot (src's offset from a 16-byte boundary).  Only keys of
+// the side's array [begin, end) are read.
+template <class T>
+__device__ __forceinline__ void merge_stage_chunk(T *slots, int c, const T *src, int chunk, const T *begin,
+                                                  const T *end) {
+  const char *p = reinterpret_cast<const char *>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(15)) + 16ll * chunk;
+  const unsigned d = (unsigned)__cvta_generic_to_shared(reinterpret_cast<uint4 *>(slots) + c);
+  if (p >= reinterpret_cast<const char *>(begin) && p + 16 <= reinterpret_cast<const char *>(end)) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; i += (int)sizeof(T)) {
+      const char *e = p + i;
+      if (e >= reinterpret_cast<const char *>(begin) && e < reinterpret_cast<const char *>(end))
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d + i), "l"(e), "n"((int)sizeof(T)) : "memory");
+    }
+  }
+}
+
+// Persistent blocks: a block's next tile is on its way into the other buffer
+// while it merges the one it holds.
+template <class T, bool DESC>
+__global__ void __launch_bounds__(MergeNet<T>::kThreads, MergeNet<T>::kBlocksPerSm)
+    merge_keys_kernel(const T *a, long long na, const T *b, long long nb, T *out, long long ntiles,
+                      const long long *splits) {
+  constexpr int ITEMS = MergeNet<T>::kItems, N = ITEMS + 1, NT = MergeNet<T>::kThreads, TILE = MergeNet<T>::kTile,
+                SLOTS = MergeNet<T>::kSlots, IPV = 16 / (int)sizeof(T);
+  static_assert(TILE % IPV == 0 && SLOTS % IPV == 0, "tiles and buffers start on 16-byte boundaries");
+  using K = KeyOrder<T, DESC>;
+  __shared__ __align__(16) T buf[2 * SLOTS];
+  __shared__ int s_lo[NT + 1];
+  const K comp;
+  const int t = threadIdx.x;
+  const long long total = na + nb;
+  const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+
+  // the tile's keys of a: [i0, i1)
+  auto range = [&](long long tile, long long &i0, long long &i1) {
+    if (tile >= ntiles) return;
+    i0 = splits[tile];
+    i1 = tile + 1 < ntiles ? splits[tile + 1] : na;
+  };
+  // start staging a tile; where its sides are: na_t keys of a from slot a0, the
+  // others of its cnt keys from slot b0
+  auto stage = [&](T *slots, long long tile, long long i0, long long i1, int &na_t, int &cnt, int &a0, int &b0) {
+    const long long d0 = tile * TILE;
+    cnt = (int)min((long long)TILE, total - d0);
+    // (the bounds hold by themselves for sorted inputs; for others they keep
+    // every access inside the inputs and the tile)
+    na_t = (int)min(max(i1 - i0, max(0ll, cnt - (nb - (d0 - i0)))), min((long long)cnt, na - i0));
+    const T *pa = a + i0, *pb = b + (d0 - i0);
+    a0 = (int)(reinterpret_cast<uintptr_t>(pa) & 15) / (int)sizeof(T);
+    const int shift_b = (int)(reinterpret_cast<uintptr_t>(pb) & 15) / (int)sizeof(T);
+    const int ca = (a0 + na_t + IPV - 1) / IPV, cb = (shift_b + (cnt - na_t) + IPV - 1) / IPV;
+    b0 = ca * IPV + shift_b;
+    for (int c = t; c < ca + cb; c += NT)
+      merge_stage_chunk(slots, c, c < ca ? pa : pb, c < ca ? c : c - ca, c < ca ? a : b, c < ca ? a + na : b + nb);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  long long tile = blockIdx.x, i0 = 0, i1 = 0;
+  int na_n = 0, cnt_n = 0, a0_n = 0, b0_n = 0;
+  range(tile, i0, i1);
+  stage(buf, tile, i0, i1, na_n, cnt_n, a0_n, b0_n);
+  range(tile + gridDim.x, i0, i1);
+  T *s = buf, *other = buf + SLOTS;
+  for (; tile < ntiles; tile += gridDim.x) {
+    const int na_t = na_n, cnt = cnt_n, nb_t = cnt_n - na_n;
+    const T *sa = s + a0_n;
+    T *sb = s + b0_n;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the tile is staged, and the other buffer's outputs are stored
+    if (tile + gridDim.x < ntiles) {
+      stage(other, tile + gridDim.x, i0, i1, na_n, cnt_n, a0_n, b0_n);
+      range(tile + 2 * (long long)gridDim.x, i0, i1);
+    }
+    // keys of a before output d: the first in [lo, hi] that a key of b precedes
+    const int d = min(t * ITEMS, cnt);
+    int lo = max(0, d - nb_t);
+    {
+      const int hi = min(d, na_t);  // hi - lo <= TILE / 2
+      constexpr int kTop = sizeof(T) == 4 ? 2048 : 1024;
+      static_assert(2 * kTop - 1 >= TILE / 2, "the steps reach every place");
+      const T *pa = sa + lo, *pb = sb + (d - 1 - lo);
+#pragma unroll
+      for (int step = kTop; step > 0; step /= 2) {
+        if (lo + step <= hi && !comp(pb[1 - step], pa[step - 1])) {
+          lo += step;
+          pa += step;
+          pb -= step;
+        }
+      }
+    }
+    s_lo[t] = lo;
+    if (t == 0) {
+      s_lo[NT] = na_t;
+      sb[nb_t] = K::last_key();
+    }
+    __syncthreads();
+    const int ca = s_lo[t + 1] - lo;
+    T v[N];
+    bool serial = d + ITEMS > cnt;
+    if (!serial) {
+      const T *pa = sa + lo, *pb = sb + (d - lo + ITEMS);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        v[i] = *(i < ca ? pa + i : pb - i);
+        serial |= K::special(v[i]);
+      }
+#pragma unroll
+      for (int h = N / 2; h > 0; h >>= 1) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          if (i & h) continue;
+          const T x = v[i], y = v[i + h];
+          v[i] = K::first(x, y);
+          v[i + h] = K::second(x, y);
+        }
+      }
+    }
+    if (serial) {
+      int ia = lo, ib = d - lo;
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const T x = sa[min(ia, na_t)], y = sb[min(ib, nb_t)];
+        const bool take_b = ib < nb_t && (ia >= na_t || comp(y, x));
+        v[k] = take_b ? y : x;
+        ia += !take_b;
+        ib += take_b;
+      }
+    }
+    __syncthreads();  // every key is read
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) s[t * ITEMS + k] = v[k];
+    __syncthreads();
+    T *o = out + tile * TILE;
+    if (cnt == TILE && vec) {
+#pragma unroll
+      for (int q = t; q < TILE / IPV; q += NT)
+        st_stream_v4(reinterpret_cast<uint4 *>(o) + q, reinterpret_cast<const uint4 *>(s)[q]);
+    } else {
+      for (int k = t; k < cnt; k += NT) o[k] = s[k];
+    }
+    T *const x = s;
+    s = other;
+    other = x;
+  }
+}
+
 // ------------------------------------------------------------------ host
 
 // Scratch of a merge of `total` keys: the tile starts.
@@ -334,6 +606,32 @@ int launch_merge(const T *a, size_t na, const T *b, size_t nb, T *out, const Com
       a, (long long)na, b, (long long)nb, total, tiles, splits, comp);
   merge_kernel<T, Comp, false><<<(unsigned)tiles, kMergeThreads, 0, st>>>(a, (long long)na, b, (long long)nb, out,
                                                                           total, splits, comp);
+  return cudaGetLastError() == cudaSuccess ? B2P_OK : B2P_ERR_CUDA;
+}
+
+// The same for standard keys, ascending or descending.
+constexpr long long kMergeWarpTiles = 4096;
+
+template <class T, bool DESC>
+int launch_merge_keys(const T *a, size_t na, const T *b, size_t nb, T *out, void *scratch, size_t scratch_bytes,
+                      int sm_count, cudaStream_t st) {
+  const long long total = (long long)(na + nb);
+  if (total == 0) return B2P_OK;
+  const long long tiles = (total + MergeNet<T>::kTile - 1) / MergeNet<T>::kTile;
+  if (tiles > 0x7fffffffLL / 32) return B2P_ERR_INVALID_ARG;
+  if (!scratch || scratch_bytes < merge_scratch_bytes<T>((size_t)total) - 256) return B2P_ERR_SCRATCH;
+  long long *splits = reinterpret_cast<long long *>(scratch);
+  // a search per warp while the tiles are few (one wave of warps: latency), 32
+  // tiles a warp beyond
+  if (tiles <= kMergeWarpTiles)
+    merge_keys_partition_kernel<T, DESC, 1><<<(unsigned)((tiles + 3) / 4), 128, 0, st>>>(a, (long long)na, b,
+                                                                                        (long long)nb, tiles, splits);
+  else
+    merge_keys_partition_kernel<T, DESC, 32><<<(unsigned)((tiles + 127) / 128), 128, 0, st>>>(
+        a, (long long)na, b, (long long)nb, tiles, splits);
+  const long long grid = std::min<long long>(tiles, (long long)sm_count * MergeNet<T>::kBlocksPerSm);
+  merge_keys_kernel<T, DESC><<<(unsigned)grid, MergeNet<T>::kThreads, 0, st>>>(a, (long long)na, b, (long long)nb, out,
+                                                                               tiles, splits);
   return cudaGetLastError() == cudaSuccess ? B2P_OK : B2P_ERR_CUDA;
 }
 

@@ -209,3 +209,47 @@ def test_radix_tile_edges(dev, code, offset):
             t.copy_(dev_t(x))
             C.sort_(t, descending=desc)
             assert same_bits(t.cpu().numpy(), O.sort(x, desc)), (n, kind)
+
+
+@pytest.mark.parametrize("code", [C.F32, C.I64])
+def test_merge_many_tiles(dev, code):
+    """More than 4096 tiles, where a partition warp takes 32 of them: the sum of
+    the keys kept and the result sorted, for sides of very different length
+    and an odd number of tiles."""
+    n = 4100 * (4960 if code == C.F32 else 2400) + 77
+    for na in (1000, n // 3):
+        g = torch.Generator(device="cuda").manual_seed(na)
+        x = torch.randint(-(1 << 23), 1 << 23, (n,), generator=g, device="cuda")
+        x = x.to(torch.float32 if code == C.F32 else torch.int64)
+        a, b = torch.sort(x[:na])[0], torch.sort(x[na:])[0]
+        assert torch.equal(C.merge(a, b), torch.sort(x)[0])
+
+
+@pytest.mark.parametrize("code", DT)
+@pytest.mark.parametrize("desc", [False, True])
+def test_merge_tile_edges(dev, code, desc):
+    """Around the merge's tiles (4960 4-byte or 2400 8-byte keys) with one side
+    empty, short or equal, unaligned output, sides that do not interleave at
+    all, the type's extreme keys$
+    sides' sentinel) and infinities among the keys, and both zeros (the
+    serial tiles)."""
+    rng = np.random.default_rng(500 + code + 10 * desc)
+    tile = 4960 if NP[code]().itemsize == 4 else 2400
+    flt = code in (C.F32, C.F64)
+    last = [np.inf, -np.inf] if flt else [np.iinfo(NP[code]).max, np.iinfo(NP[code]).min]
+    for total in (tile - 1, tile, tile + 1, 8 * tile, 8 * tile + 1, 16 * tile - 1):
+        for na in (0, 1, 31, total // 2, total - 16, total):
+            for kind in ("random", "dup", "last", "apart"):
+                x = keys(rng, code, total, kind == "dup")
+                if kind == "last":
+                    x[rng.random(total) < 0.3] = last[0]
+                    x[rng.random(total) < 0.3] = last[1]
+                if kind == "apart":
+                    x.sort()
+                    if (total + na) % 2:
+                        x = x[::-1]
+                a, b = O.sort(x[:na].copy(), desc), O.sort(x[na:].copy(), desc)
+                off = total % 2
+                out = torch.empty(total + off, dtype=dev_t(x[:1].copy()).dtype, device="cuda")[off:]
+                C.merge(dev_t(a), dev_t(b), out=out, descending=desc)
+                assert same_bits(out.cpu().numpy(), O.merge(a, b, desc)), (total, na, kind)
