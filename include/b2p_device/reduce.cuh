@@ -143,79 +143,135 @@ __device__ __forceinline__ void fold(typename P::Acc &acc, typename P::In a, typ
   }
 }
 
+// Compensated folds keep kFoldChains accumulators (element e of each vector
+// goes to chain e % kFoldChains: two for fp32, four for bf16), shortening the
+// dependent TwoSum chain; the order depends only on element positions, so
+// every launch configuration gives the same bits.
+//
+// The value of one run (all lanes of its warp; every lane returns it), with B
+// 16-byte loads in flight per lane.
 template <class P, bool DOT, bool VEC>
-__global__ void __launch_bounds__(1024) reduce_kernel(ReduceParams p) {
+__device__ __forceinline__ typename P::Acc fold_run(const ReduceParams &p, long long run, int B) {
   using In = typename P::In;
   using Acc = typename P::Acc;
   using VT = typename VecOf<In, VEC>::type;
   constexpr int V = VecOf<In, VEC>::kElems;
   constexpr int kMaxB = (DOT || sizeof(In) == 8) ? 4 : 8;
+  constexpr int kChains = !P::kCompensated || V == 1 ? 1 : (V >= 8 ? 4 : 2);
+  const In *a = reinterpret_cast<const In *>(p.a) + p.head;
+  const In *b = DOT ? reinterpret_cast<const In *>(p.b) + p.head : nullptr;
+  const long long nvec = (long long)p.nvec;
+  B = min(B, kMaxB);
+  Acc acc[kChains];
+#pragma unroll
+  for (int c = 0; c < kChains; ++c) acc[c] = P::identity();
+  const long long base = run * 32LL * p.K + (threadIdx.x & 31);
+  for (int j0 = 0; j0 < p.K; j0 += B) {
+    const long long v0 = base + (long long)j0 * 32;
+    if (v0 + (long long)(B - 1) * 32 < nvec) {
+      // whole batch in range: B independent 16-byte loads in flight
+      VT va[kMaxB], vb[kMaxB];
+#pragma unroll
+      for (int k = 0; k < kMaxB; ++k)
+        if (k < B) {
+          va[k] = load_vec<In, VEC>(a, v0 + k * 32);
+          if constexpr (DOT) vb[k] = load_vec<In, VEC>(b, v0 + k * 32);
+        }
+#pragma unroll
+      for (int k = 0; k < kMaxB; ++k)
+        if (k < B) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            In xa = vec_elem<In>(va[k], e);
+            In xb = DOT ? vec_elem<In>(vb[k], e) : xa;
+            fold<P, DOT>(acc[e % kChains], xa, xb);
+          }
+        }
+    } else {
+      // ragged end of the last run
+      for (int k = 0; k < B; ++k) {
+        const long long vi = v0 + k * 32;
+        if (vi < nvec) {
+          VT xa = load_vec<In, VEC>(a, vi);
+          VT xb = xa;
+          if constexpr (DOT) xb = load_vec<In, VEC>(b, vi);
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            fold<P, DOT>(acc[e % kChains], vec_elem<In>(xa, e), DOT ? vec_elem<In>(xb, e) : vec_elem<In>(xa, e));
+        }
+      }
+    }
+  }
+  if constexpr (kChains == 4) {
+    acc[0] = P::combine(acc[0], acc[1]);
+    acc[2] = P::combine(acc[2], acc[3]);
+  }
+  if constexpr (kChains >= 2) acc[0] = P::combine(acc[0], acc[kChains / 2]);
+  Acc r = acc[0];
+  if constexpr (P::kCompensated) r = df_norm(r);
+  return warp_allreduce<P>(r);
+}
 
+// The elements before the aligned body and after it (fewer than 16 bytes
+// each), loaded by the lanes of one warp and folded in order; every lane
+// returns both values.
+template <class P, bool DOT, bool VEC>
+struct ReduceEnds {
+  using In = typename P::In;
+  using Acc = typename P::Acc;
+  In ha, hb, ta, tb;  // this lane's element of the head and of the tail
+  __device__ __forceinline__ ReduceEnds(const ReduceParams &p) {
+    const unsigned lane = threadIdx.x & 31;
+    const In *a = reinterpret_cast<const In *>(p.a), *b = reinterpret_cast<const In *>(p.b);
+    const unsigned long long ts = p.head + p.nvec * VecOf<In, VEC>::kElems;
+    ha = hb = ta = tb = In{};
+    if (lane < p.head) {
+      ha = a[lane];
+      if constexpr (DOT) hb = b[lane];
+    }
+    if (lane < p.tail) {
+      ta = a[ts + lane];
+      if constexpr (DOT) tb = b[ts + lane];
+    }
+  }
+  __device__ __forceinline__ static In lane_value(In v, int i) {
+    if constexpr (sizeof(In) == 2) return (In)__shfl_sync(0xffffffffu, (unsigned)v, i);
+    else return shfl_idx(v, i);
+  }
+  __device__ __forceinline__ void fold_in_order(const ReduceParams &p, Acc &h, Acc &t) const {
+    h = P::identity();
+    t = P::identity();
+    for (int i = 0; i < (int)p.head; ++i) fold<P, DOT>(h, lane_value(ha, i), lane_value(DOT ? hb : ha, i));
+    for (int i = 0; i < (int)p.tail; ++i) fold<P, DOT>(t, lane_value(ta, i), lane_value(DOT ? tb : ta, i));
+    if constexpr (P::kCompensated) {
+      h = df_norm(h);
+      t = df_norm(t);
+    }
+  }
+};
+
+// *out = op(init or *out, head + body + tail), by one thread.
+template <class P>
+__device__ __forceinline__ void write_total(const ReduceParams &p, typename P::Acc head, typename P::Acc body,
+                                            typename P::Acc tail) {
+  using Out = typename P::Out;
+  const typename P::Acc total = P::combine(P::combine(head, body), tail);
+  Out *out = reinterpret_cast<Out *>(p.out);
+  const Out basev = p.has_init ? from_bits64<Out>(p.init_bits) : *out;
+  *out = P::finalize(P::combine(P::from_out(basev), total));
+}
+
+template <class P, bool DOT, bool VEC>
+__global__ void __launch_bounds__(1024) reduce_kernel(ReduceParams p) {
+  using Acc = typename P::Acc;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
   const long long gw = (long long)blockIdx.x * wpb + warp;
   const long long tw = (long long)gridDim.x * wpb;
-  const In *a = reinterpret_cast<const In *>(p.a) + p.head;
-  const In *b = DOT ? reinterpret_cast<const In *>(p.b) + p.head : nullptr;
-  const long long nvec = (long long)p.nvec;
-  const int B = min(p.B, kMaxB);
   const unsigned long long epoch = *reinterpret_cast<volatile unsigned long long *>(&p.hdr->epoch);
-
-  // Compensated folds keep kChains accumulators (element e of each vector
-  // goes to chain e % kChains: two for fp32, four for bf16), shortening the
-  // dependent TwoSum chain; the order depends only on element positions, so
-  // every launch configuration gives the same bits.
-  constexpr int kChains = !P::kCompensated || V == 1 ? 1 : (V >= 8 ? 4 : 2);
   for (long long run = gw; run < p.runs; run += tw) {
-    Acc acc[kChains];
-#pragma unroll
-    for (int c = 0; c < kChains; ++c) acc[c] = P::identity();
-    const long long base = run * 32LL * p.K + lane;
-    for (int j0 = 0; j0 < p.K; j0 += B) {
-      const long long v0 = base + (long long)j0 * 32;
-      if (v0 + (long long)(B - 1) * 32 < nvec) {
-        // whole batch in range: B independent 16-byte loads in flight
-        VT va[kMaxB], vb[kMaxB];
-#pragma unroll
-        for (int k = 0; k < kMaxB; ++k)
-          if (k < B) {
-            va[k] = load_vec<In, VEC>(a, v0 + k * 32);
-            if constexpr (DOT) vb[k] = load_vec<In, VEC>(b, v0 + k * 32);
-          }
-#pragma unroll
-        for (int k = 0; k < kMaxB; ++k)
-          if (k < B) {
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-              In xa = vec_elem<In>(va[k], e);
-              In xb = DOT ? vec_elem<In>(vb[k], e) : xa;
-              fold<P, DOT>(acc[e % kChains], xa, xb);
-            }
-          }
-      } else {
-        // ragged end of the last run
-        for (int k = 0; k < B; ++k) {
-          const long long vi = v0 + k * 32;
-          if (vi < nvec) {
-            VT xa = load_vec<In, VEC>(a, vi);
-            VT xb = xa;
-            if constexpr (DOT) xb = load_vec<In, VEC>(b, vi);
-#pragma unroll
-            for (int e = 0; e < V; ++e)
-              fold<P, DOT>(acc[e % kChains], vec_elem<In>(xa, e), DOT ? vec_elem<In>(xb, e) : vec_elem<In>(xa, e));
-          }
-        }
-      }
-    }
-    if constexpr (kChains == 4) {
-      acc[0] = P::combine(acc[0], acc[1]);
-      acc[2] = P::combine(acc[2], acc[3]);
-    }
-    if constexpr (kChains >= 2) acc[0] = P::combine(acc[0], acc[kChains / 2]);
-    Acc r = acc[0];
-    if constexpr (P::kCompensated) r = df_norm(r);
-    r = warp_allreduce<P>(r);
+    const Acc r = fold_run<P, DOT, VEC>(p, run, p.B);
     if (lane == 0) st_status(p.partials + run, P::pack(r), (epoch << 8) | kFlagAgg);
   }
 
@@ -223,26 +279,50 @@ __global__ void __launch_bounds__(1024) reduce_kernel(ReduceParams p) {
   __shared__ unsigned long long s_v[kFinalWidth];
   if (!last_block_arrives(p.hdr)) return;
   combine_run_partials<P>(p.partials, p.runs, s_v);
-  if (threadIdx.x == 0) {
-    const In *a0 = reinterpret_cast<const In *>(p.a);
-    const In *b0 = reinterpret_cast<const In *>(p.b);
-    Acc h = P::identity();
-    for (unsigned long long i = 0; i < p.head; ++i) fold<P, DOT>(h, a0[i], DOT ? b0[i] : a0[i]);
-    Acc t = P::identity();
-    const unsigned long long ts = p.head + p.nvec * V;
-    for (unsigned long long i = ts; i < ts + p.tail; ++i) fold<P, DOT>(t, a0[i], DOT ? b0[i] : a0[i]);
-    if constexpr (P::kCompensated) {
-      h = df_norm(h);
-      t = df_norm(t);
+  if (warp == 0) {
+    const ReduceEnds<P, DOT, VEC> ends(p);
+    Acc h, t;
+    ends.fold_in_order(p, h, t);
+    if (lane == 0) {
+      write_total<P>(p, h, P::unpack(s_v[0]), t);
+      // every block read the epoch before arriving; the next launch sees this
+      atomicAdd(&p.hdr->epoch, 1ull);
     }
-    Acc total = P::combine(P::combine(h, P::unpack(s_v[0])), t);
-    using Out = typename P::Out;
-    Out *out = reinterpret_cast<Out *>(p.out);
-    Out basev = p.has_init ? from_bits64<Out>(p.init_bits) : *out;
-    *out = P::finalize(P::combine(P::from_out(basev), total));
-    // every block read the epoch before arriving; the next launch sees this
-    atomicAdd(&p.hdr->epoch, 1ull);
   }
+}
+
+// At most 32 runs (256 KiB of input): one block, a warp per run, whose values
+// meet in shared memory instead of going through status words, a fence and
+// the arrival counter in global memory (four round trips to L2).  The same
+// tree as combine_run_partials: slot v of kFinalWidth is identity (+) run v,
+// then halves are combined; slots from 32 on hold the identity.
+// A reduce of 1,021 int32 takes 2.9 us this way, 6.0 us through reduce_kernel.
+constexpr int kSmallRuns = 32;
+
+template <class P, bool DOT, bool VEC>
+__global__ void __launch_bounds__(32 * kSmallRuns) reduce_small_kernel(ReduceParams p) {
+  using Acc = typename P::Acc;
+  __shared__ unsigned long long s_run[kSmallRuns];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const ReduceEnds<P, DOT, VEC> ends(p);
+  if (warp < p.runs) {
+    const Acc r = fold_run<P, DOT, VEC>(p, warp, 8);
+    if (lane == 0) s_run[warp] = P::pack(r);
+  }
+  __syncthreads();
+  if (warp > 0) return;
+  Acc v = P::identity();
+  if (lane < p.runs) v = P::combine(v, P::unpack(s_run[lane]));
+#pragma unroll
+  for (int w = kFinalWidth / 2; w >= kSmallRuns; w >>= 1) v = P::combine(v, P::identity());
+#pragma unroll
+  for (int w = kSmallRuns / 2; w >= 1; w >>= 1) {
+    const Acc o = shfl_idx(v, (lane + w) & 31);
+    if (lane < w) v = P::combine(v, o);
+  }
+  Acc h, t;
+  ends.fold_in_order(p, h, t);
+  if (lane == 0) write_total<P>(p, h, v, t);
 }
 
 

@@ -53,19 +53,21 @@ int launch_t(const void *a, const void *b, size_t n, void *out, const void *init
   if (init) memcpy(&p.init_bits, init, sizeof(typename P::Out));
   p.hdr = reinterpret_cast<ScratchHeader *>(scratch);
   p.partials = reinterpret_cast<StatusWord *>(reinterpret_cast<char *>(scratch) + kScratchPrefix);
-  int wpb = lc.block / 32;
-  if constexpr (DOT) {
-    if (!sh.vec) {
-      const void *kfn = (const void *)reduce_kernel<P, DOT, false>;
-      int grid = grid_for(lc.grid_mode, std::max<long long>(sh.runs, 1), wpb, kfn, lc.block, 0);
-      reduce_kernel<P, DOT, false><<<grid, lc.block, 0, st>>>(p);
+  auto launch = [&](auto vec) {
+    constexpr bool VEC = decltype(vec)::value;
+    if (sh.runs <= kSmallRuns) {
+      reduce_small_kernel<P, DOT, VEC><<<1, 32 * (int)std::max<long long>(sh.runs, 1), 0, st>>>(p);
       return cuda_status(cudaGetLastError());
     }
+    const void *kfn = (const void *)reduce_kernel<P, DOT, VEC>;
+    int grid = grid_for(lc.grid_mode, sh.runs, lc.block / 32, kfn, lc.block, 0);
+    reduce_kernel<P, DOT, VEC><<<grid, lc.block, 0, st>>>(p);
+    return cuda_status(cudaGetLastError());
+  };
+  if constexpr (DOT) {
+    if (!sh.vec) return launch(std::false_type{});
   }
-  const void *kfn = (const void *)reduce_kernel<P, DOT, true>;
-  int grid = grid_for(lc.grid_mode, std::max<long long>(sh.runs, 1), wpb, kfn, lc.block, 0);
-  reduce_kernel<P, DOT, true><<<grid, lc.block, 0, st>>>(p);
-  return cuda_status(cudaGetLastError());
+  return launch(std::true_type{});
 }
 
 template <int DT>
@@ -99,8 +101,9 @@ int dispatch_op(int op, const void *a, const void *b, size_t n, void *out, const
 template <int DT, int OP>
 int preload_one() {
   cudaFuncAttributes fa;
-  cudaError_t e =
-      cudaFuncGetAttributes(&fa, (const void *)reduce_kernel<typename PolicyOf<DT, OP>::type, false, true>);
+  using P = typename PolicyOf<DT, OP>::type;
+  cudaError_t e = cudaFuncGetAttributes(&fa, (const void *)reduce_kernel<P, false, true>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void *)reduce_small_kernel<P, false, true>);
   return cuda_status(e);
 }
 

@@ -472,3 +472,38 @@ def test_kernels_are_sm100a(dev):
     b, p = ctypes.c_int(0), ctypes.c_int(-1)
     C.check(C.lib().b2p_kernel_arch(ctypes.byref(b), ctypes.byref(p)), "b2p_kernel_arch")
     assert b.value == 100, b.value
+
+
+@pytest.mark.parametrize("code", [C.I32, C.I64, C.F32, C.BF16, C.F64])
+def test_reduce_one_block_limit(dev, code):
+    """Sizes on both sides of the one-block reduce's limit (32 runs of 8 KiB),
+    of a run, of a vector, and starts up to seven elements off a 16-byte
+    boundary: integers exact, floats within 1e-6 of the FP64 sum, the same bits
+    in every launch configuration; combining with *out; the dot product."""
+    es = {C.I32: 4, C.I64: 8, C.F32: 4, C.BF16: 2, C.F64: 8}[code]
+    run = 8192 // es
+    g = torch.Generator(device="cuda").manual_seed(code)
+    for n in (1, 2, 16 // es, run - 1, run, run + 1, 32 * run - 1, 32 * run, 32 * run + 1, 33 * run + 5):
+        for off in (0, 1, 3):
+            if code in (C.I32, C.I64):
+                base = torch.randint(-1000, 1000, (n + off,), generator=g, device="cuda")
+                x = base.to(torch.int32 if code == C.I32 else torch.int64)[off:]
+            else:
+                base = torch.randn(n + off, generator=g, device="cuda", dtype=torch.float64)
+                x = base.to({C.F32: torch.float32, C.BF16: torch.bfloat16, C.F64: torch.float64}[code])[off:]
+            ref = x.to(torch.float64).sum().item()
+            scale = x.to(torch.float64).abs().sum().item()
+            bits = set()
+            for cfg in (C.AUTO, 0, 15, 17, 47):
+                got = C.reduce(x, "sum", init=0, config=cfg)
+                bits.add(got.view(torch.uint8).cpu().numpy().tobytes())
+                assert abs(got.item() - ref) <= 1e-6 * abs(ref) + 1e-12 * scale, (n, off, cfg)
+            assert len(bits) == 1, (n, off)
+            if code in (C.I32, C.I64):
+                assert C.reduce(x, "min", init=5).item() == min(5, int(x.min()))
+                keep = torch.full((1,), 7, dtype=x.dtype, device="cuda")
+                assert C.reduce(x, "sum", init=None, out=keep).item() == 7 + int(x.sum())
+            else:
+                d = C.dot(x, x, init=1.0).item()
+                rd = 1.0 + (x.to(torch.float64) ** 2).sum().item()
+                assert abs(d - rd) <= 1e-6 * rd, (n, off)
