@@ -49,6 +49,7 @@ struct ScanParams {
   int vec_out;                   // output 16-byte aligned
   ScratchHeader *hdr;
   StatusWord *status;            // one word per tile
+  int fixed_ids;                 // look-back kernels: block b takes tile b, and no other
   StatusWord *chunk_status;      // two-phase: chunk totals / inclusive prefixes (look-back)
   StatusWord *chunk_carry;       // two-phase: exclusive carry of each chunk
   unsigned *counters;            // two-phase: phase-1 arrivals per chunk
@@ -180,6 +181,17 @@ __device__ void finalize_chunk(const ScanParams &p, long long k, unsigned long l
 
 // ---------------------------------------------------------- scan kernels
 
+// The block's next tile of a look-back kernel: the next dynamic id, so that a
+// tile's predecessors have always started, or, when every block of the launch
+// fits on the GPU at once, the block's own index (a ticket is a round trip to
+// L2 before the first load, and another one to learn that there are no more).
+__device__ __forceinline__ long long next_tile(const ScanParams &p, unsigned long long *s_tile) {
+  if (p.fixed_ids) return blockIdx.x;
+  if (threadIdx.x == 0) *s_tile = atomicAdd(&p.hdr->tile_ctr, 1ull);
+  __syncthreads();
+  return (long long)*s_tile;
+}
+
 template <class P, int ITEMS, bool WIDE>
 __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
     scan_lookback_kernel(ScanParams p) {
@@ -203,20 +215,16 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
   const unsigned long long pol = l2_policy_stream();
 
   if (threadIdx.x == 0) s_epoch = *reinterpret_cast<volatile unsigned long long *>(&p.hdr->epoch);
-  __syncthreads();
-  const unsigned long long epoch = s_epoch;
-  const unsigned long long epoch_tag = epoch << 8;
   const unsigned long long init_bits = init_value<P, WIDE>(p);
 
   while (true) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&p.hdr->tile_ctr, 1ull);
-    __syncthreads();
-    const long long tile = (long long)s_tile;
+    const long long tile = next_tile(p, &s_tile);
     if (tile >= p.ntiles) break;
     const unsigned long long base = (unsigned long long)tile * tile_elems;
     const int count = (int)min((unsigned long long)tile_elems, p.n - base);
     load_tile_smem<In>(buf, in + base, count, tile_elems, p.vec_in, pol);
     __syncthreads();
+    const unsigned long long epoch_tag = s_epoch << 8;
 
     const Acc agg = thread_total<P, ITEMS>(buf, count);
     Acc tile_agg;
@@ -247,9 +255,10 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
     emit_scan<P, ITEMS>(buf, obuf, start_value<P, WIDE>(s_carry, texcl), p.inclusive);
     __syncthreads();
     store_tile<Out>(obuf, out + base, count, tile_elems, p.vec_out);
+    if (p.fixed_ids) break;
     __syncthreads();
   }
-  finish_launch(p.hdr, epoch, nullptr, 0);
+  finish_launch(p.hdr, s_epoch, nullptr, 0);
 }
 
 template <class P, int ITEMS, bool WIDE>
@@ -425,19 +434,15 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
   const unsigned long long pol = l2_policy_stream();
 
   if (threadIdx.x == 0) s_epoch = *reinterpret_cast<volatile unsigned long long *>(&p.hdr->epoch);
-  __syncthreads();
-  const unsigned long long epoch = s_epoch;
-  const unsigned long long epoch_tag = epoch << 8;
 
   while (true) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(&p.hdr->tile_ctr, 1ull);
-    __syncthreads();
-    const long long tile = (long long)s_tile;
+    const long long tile = next_tile(p, &s_tile);
     if (tile >= p.ntiles) break;
     const unsigned long long base = (unsigned long long)tile * tile_elems;
     const int count = (int)min((unsigned long long)tile_elems, p.n - base);
     load_tile_smem<T>(buf, in + base, count, tile_elems, p.vec_in, pol);
     __syncthreads();
+    const unsigned long long epoch_tag = s_epoch << 8;
     int kept;
     const unsigned keep = thread_flags<T, ITEMS>(buf, count, p, &kept);
     unsigned long long tile_kept;
@@ -474,9 +479,10 @@ __global__ void __launch_bounds__(ITEMS <= 8 ? 1024 : 8192 / ITEMS)
     } else if (threadIdx.x == 0) {
       record_error(p.hdr, B2P_ERR_INVALID_ARG);
     }
+    if (p.fixed_ids) break;
     __syncthreads();
   }
-  finish_launch(p.hdr, epoch, nullptr, 0);
+  finish_launch(p.hdr, s_epoch, nullptr, 0);
 }
 
 template <class T, int ITEMS>
@@ -674,6 +680,8 @@ int launch_kernel(K kernel, ScanParams &p, const LaunchConfig &lc, size_t smem, 
   int rc = ensure_dynamic_smem(kfn, smem);
   if (rc) return rc;
   int grid = grid_for(lc.grid_mode, units, 1, kfn, lc.block, smem);
+  if (lc.grid_mode == 0)
+    p.fixed_ids = units <= (long long)device_info().sm_count * occupancy(kfn, lc.block, smem);
   kernel<<<grid, lc.block, smem, st>>>(p);
   return cuda_status(cudaGetLastError());
 }

@@ -41,20 +41,34 @@ int heuristic_config(int prim, int dtype, size_t n, int64_t nseg) {
     int ii = items == 4 ? 0 : items == 8 ? 1 : items == 16 ? 2 : 3;
     return grid_mode * 16 + bi * 4 + ii;
   };
-  // Fixed choices from configuration sweeps of 2^28-element inputs on B200.
+  // Fixed choices from configuration sweeps on B200 (launches back to back in a
+  // CUDA graph).
+  const size_t es = dtype_size(dtype), bytes = n * es;
   switch (prim) {
   case B2P_PRIM_REDUCE:
   case B2P_PRIM_DOT:
-    return cfg(0, 1024, 32);
+    // more, smaller blocks while the runs do not fill the GPU (2^18 floats: 23 %
+    // slower with 1024 threads)
+    return bytes <= (4u << 20) ? cfg(0, 256, 32) : bytes <= (16u << 20) ? cfg(0, 512, 32) : cfg(0, 1024, 32);
   case B2P_PRIM_SCAN:
-    // pipelined (TMA) kernel from 8 MiB of input on; below that the
-    // one-tile-per-block look-back kernel fills the GPU faster
-    if (n * dtype_size(dtype) >= (8u << 20))
-      return cfg(1, 256, dtype_size(dtype) == 8 ? 16 : 32);
-    return cfg(0, 256, dtype_size(dtype) == 8 ? 16 : 32);
-  case B2P_PRIM_COPY_IF:
-    if (n * dtype_size(dtype) >= (8u << 20)) return cfg(1, 256, dtype_size(dtype) == 8 ? 16 : 32);
-    return cfg(0, 256, dtype_size(dtype) == 8 ? 16 : 32);
+  case B2P_PRIM_COPY_IF: {
+    // The pipelined (TMA) kernel once its blocks have several tiles each: a scan
+    // beyond 16 MiB (2^22 int32: 15.5 us against 14.0 us of the look-back
+    // kernel; 2^23: 37 against 50), copy_if from 8 MiB of input on (2^21
+    // uint32: 11.2 against 14.0).
+    const bool scan = prim == B2P_PRIM_SCAN;
+    if (scan ? n * acc_size(dtype) > (16u << 20) : bytes >= (8u << 20)) return cfg(1, 256, es == 8 ? 16 : 32);
+    // Below, one look-back tile per block: the smallest tile that still leaves
+    // at most about one tile per SM, because the time is the latency of one
+    // tile and the look-back over the others (2^16 int32: 5.5 us with 2048
+    // elements, 10.5 us with 8192; 2^19: 7.2 us with 4096, 11.3 us with 8192;
+    // 2^21: 10.0 us with 512 x 16, 12.4 us with 256 x 32).
+    if (n <= (1u << 18)) return es == 2 ? cfg(0, 256, 8) : cfg(0, 512, 4);
+    if (n <= (1u << 19)) return es == 4 ? cfg(0, 1024, 4) : cfg(0, 512, 8);
+    if (scan && es == 8) return cfg(0, 256, 16);
+    if (n <= (1u << 20)) return cfg(0, 1024, 8);
+    return n <= (1u << 21) ? cfg(0, 512, 16) : cfg(0, 256, 32);
+  }
   case B2P_PRIM_HISTOGRAM:
     return cfg(1, 1024, 32);
   case B2P_PRIM_SEG_REDUCE:

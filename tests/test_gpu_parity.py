@@ -507,3 +507,29 @@ def test_reduce_one_block_limit(dev, code):
                 d = C.dot(x, x, init=1.0).item()
                 rd = 1.0 + (x.to(torch.float64) ** 2).sum().item()
                 assert abs(d - rd) <= 1e-6 * rd, (n, off)
+
+
+@pytest.mark.parametrize("code", [C.I32, C.I64, C.F32, C.BF16])
+def test_scan_and_copy_if_at_the_tile_rules(dev, code):
+    """Sizes on both sides of every size rule of the automatic configuration
+    (one look-back tile per block with its own index as tile id, then the
+    pipelined kernel): the scan against torch's cumulative sum, copy_if
+    against a mask, integers exact, floats within 1e-6."""
+    g = torch.Generator(device="cuda").manual_seed(code)
+    for n in (1, 2048, 2049, 1 << 18, (1 << 18) + 1, 1 << 19, (1 << 19) + 1, 1 << 20, (1 << 20) + 1, 1 << 21,
+              (1 << 21) + 1, 1 << 22, (1 << 22) + 1):
+        if code in (C.I32, C.I64):
+            x = torch.randint(0, 1 << 20, (n,), generator=g, device="cuda")
+            x = x.to(torch.int32 if code == C.I32 else torch.int64)
+            ref = torch.cumsum(x, 0).to(x.dtype)
+            assert torch.equal(C.inclusive_scan(x), ref), n
+            ex = C.exclusive_scan(x, 5)
+            assert ex[0].item() == 5 and torch.equal(ex[1:], ref[:-1] + 5), n
+            out, cnt = C.copy_if(x, 7, C.CMP_LT, 3)
+            keep = x[(x & 7) < 3]
+            assert int(cnt.item()) == keep.numel() and torch.equal(out[:keep.numel()], keep), n
+        else:
+            x = torch.rand(n, generator=g, device="cuda").to(torch.float32 if code == C.F32 else torch.bfloat16)
+            ref = torch.cumsum(x.to(torch.float64), 0)
+            got = C.inclusive_scan(x).to(torch.float64)
+            assert ((got - ref).abs() <= 1e-6 * ref.abs() + 1e-30).all(), n
