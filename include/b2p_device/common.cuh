@@ -40,11 +40,49 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void *p) {
   return r;
 }
 
+// The same through L2 only: for what a kernel that is still running when this
+// one starts may write (programmatic dependent launch, below).
+__device__ __forceinline__ uint4 ld_stream_l2_v4(const void *p) {
+  uint4 r;
+  asm volatile("ld.global.cg.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
 // 16-byte streaming store (evict-first): outputs are not re-read here.
 __device__ __forceinline__ void st_stream_v4(void *p, uint4 v) {
   asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y),
                "r"(v.z), "r"(v.w)
                : "memory");
+}
+
+// Programmatic dependent launch, for the short kernels of one call: a kernel
+// started by launch_dependent() is brought up while the one before it in the
+// stream still runs.  It calls grid_wait() before its first access to global
+// memory (the kernels before it are complete and their writes visible then),
+// and grid_trigger() after that, so that no more than two kernels of a stream
+// overlap.  What an earlier kernel of the chain wrote is read through L2 only
+// (__ldcg, cp.async.cg): L1 is not invalidated in between.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// early = false: an ordinary launch of such a kernel.
+template <class... P, class... A>
+inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                                    cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &attr;
+  c.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
 // Tile status word of the single-pass look-back: {payload, meta} read and

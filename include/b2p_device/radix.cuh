@@ -136,6 +136,8 @@ __global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *k
   for (unsigned i = t; i < kRadixBins * 8; i += kRadixThreads)
     reinterpret_cast<uint4 *>(sh)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
+  grid_wait();
+  grid_trigger();
   const RadixDigit<T> dg(pass, desc);
   auto count = [&](const T &k) {
     atomicAdd(reinterpret_cast<unsigned *>(reinterpret_cast<char *>(sh) + dg.template at<7>(k, lane << 2)), 1u);
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *k
     for (; i + kRadixStep <= b1; i += kRadixStep) {
       uint4 v[V];
 #pragma unroll
-      for (unsigned r = 0; r < V; ++r) v[r] = ld_stream_v4(keys + i + (r * kRadixThreads + t) * IPV);
+      for (unsigned r = 0; r < V; ++r) v[r] = ld_stream_l2_v4(keys + i + (r * kRadixThreads + t) * IPV);
 #pragma unroll
       for (unsigned r = 0; r < V; ++r) {
         T k[IPV];
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *k
       }
     }
   }
-  for (i += t; i < b1; i += kRadixThreads) count(keys[i]);
+  for (i += t; i < b1; i += kRadixThreads) count(__ldcg(keys + i));
   __syncthreads();
   for (unsigned d = t; d < kRadixBins; d += kRadixThreads) {
     unsigned c = 0;
@@ -176,7 +178,9 @@ __global__ void __launch_bounds__(kRadixSpineThreads) radix_spine_kernel(unsigne
   __shared__ unsigned s_warp[kRadixSpineThreads / 32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   unsigned *row = counts + (size_t)blockIdx.x * blocks;
-  const unsigned c = t < blocks ? row[t] : 0u;
+  grid_wait();
+  grid_trigger();
+  const unsigned c = t < blocks ? __ldcg(row + t) : 0u;
   unsigned incl = c;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -251,7 +255,7 @@ __device__ __forceinline__ void radix_load_tile(char *buf, const T *in, unsigned
   } else {
     for (unsigned e = t; e < TILE; e += kDownThreads) {
       const unsigned kb = e / K, b = (e % K) * (unsigned)sizeof(T);
-      const T x = e < count ? in[t0 + e] : pad;
+      const T x = e < count ? __ldcg(in + t0 + e) : pad;
       *reinterpret_cast<T *>(buf + radix_stage((kb & 3u) * 32u + (kb >> 2), b >> 4) + (b & 15u)) = x;
     }
   }
@@ -298,15 +302,6 @@ __global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
     return before + incl - mine.x - mine.y;
   };
 
-  // next output slot of this thread's digits 2t and 2t + 1 in this chunk
-  uint2 mine;
-  s_tot[2 * t] = totals[2 * t];
-  s_tot[2 * t + 1] = totals[2 * t + 1];
-  __syncthreads();
-  unsigned run0 = start_of(mine), run1 = run0 + mine.x;
-  run0 += prefix[(size_t)(2 * t) * gridDim.x + blockIdx.x];
-  run1 += prefix[(size_t)(2 * t + 1) * gridDim.x + blockIdx.x];
-
   const unsigned ntiles = (n + TILE - 1) / TILE;
   const unsigned tile_begin = (unsigned)(blockIdx.x * chunk);
   const unsigned tile_end = min(ntiles, tile_begin + (unsigned)chunk);
@@ -325,11 +320,25 @@ __global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
   const unsigned b_lt = q < (g >> 1) ? ones : 0u, b_le = q <= (g >> 1) ? ones : 0u,
                  b_mid = (g & 1u) ? b_le : b_lt;
 
-  if (tile_begin < tile_end)
-    radix_load_tile<T>(x, in, tile_begin * TILE, min(TILE, n - tile_begin * TILE), vec, pad);
 #pragma unroll
   for (int i = 0; i < kRadixTileBytes / (kDownThreads * 16); ++i)
     *reinterpret_cast<uint4 *>(y + (i * kDownThreads + t) * 16) = make_uint4(0, 0, 0, 0);
+  grid_wait();
+  grid_trigger();
+  if (tile_begin < tile_end)
+    radix_load_tile<T>(x, in, tile_begin * TILE, min(TILE, n - tile_begin * TILE), vec, pad);
+
+  // next output slot of this thread's digits 2t and 2t + 1 in this chunk
+  uint2 mine;
+  unsigned run0 = __ldcg(prefix + (size_t)(2 * t) * gridDim.x + blockIdx.x),
+           run1 = __ldcg(prefix + (size_t)(2 * t + 1) * gridDim.x + blockIdx.x);
+  *reinterpret_cast<uint2 *>(s_tot + 2 * t) = __ldcg(reinterpret_cast<const uint2 *>(totals) + t);
+  __syncthreads();
+  {
+    const unsigned start = start_of(mine);
+    run0 += start;
+    run1 += start + mine.x;
+  }
 
   for (unsigned tile = tile_begin; tile < tile_end; ++tile) {
     const unsigned count = min(TILE, n - tile * TILE);
@@ -497,13 +506,21 @@ int launch_radix_sort(T *keys, size_t n, bool desc, void *scratch, size_t scratc
   if (cudaFuncSetAttribute((const void *)radix_downsweep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return B2P_ERR_CUDA;
+  // One tile per block: 3 P launches of 3 to 10 us each, which overlap their
+  // start with the end of the one before (1,000,003 doubles: 156 -> 144 us).
+  // Longer launches start in order: early blocks of the next kernel keep an SM
+  // from taking its share (2^28 int32: 3.81 ms against 4.18).
+  const bool early = l.chunk == 1;
   const T *src = keys;
   T *dst = buf;
   for (int p = 0; p < P; ++p) {
-    radix_upsweep_kernel<T><<<l.blocks, kRadixThreads, 0, st>>>(src, (unsigned)n, desc, p, l.chunk, counts);
-    radix_spine_kernel<<<kRadixBins, kRadixSpineThreads, 0, st>>>(counts, l.blocks, totals);
-    radix_downsweep_kernel<T><<<l.blocks, kDownThreads, smem, st>>>(src, dst, (unsigned)n, desc, p, l.chunk, counts,
-                                                                    totals, radix_pad<T>(desc));
+    if (launch_dependent(early, radix_upsweep_kernel<T>, l.blocks, kRadixThreads, 0, st, src, (unsigned)n, desc, p, l.chunk,
+                         counts) != cudaSuccess ||
+        launch_dependent(early, radix_spine_kernel, kRadixBins, kRadixSpineThreads, 0, st, counts, l.blocks, totals) !=
+            cudaSuccess ||
+        launch_dependent(early, radix_downsweep_kernel<T>, l.blocks, kDownThreads, smem, st, src, dst, (unsigned)n, desc, p,
+                         l.chunk, counts, totals, radix_pad<T>(desc)) != cudaSuccess)
+      return B2P_ERR_CUDA;
     src = dst;
     dst = (dst == buf) ? keys : buf;
   }
