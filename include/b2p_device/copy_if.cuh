@@ -58,40 +58,73 @@ __device__ __forceinline__ unsigned keep_bits(const uint32_t *w, const Pred &pre
   for (int j = 0; j < ITEMS; ++j) {
     T e;
     memcpy(&e, w + j * (int)(sizeof(T) / 4), sizeof(T));
-    keep |= (unsigned)static_cast<bool>(pred(e)) << j;
+    if (pred(e)) keep |= 1u << j;
   }
   if (count < first + ITEMS) keep &= count <= first ? 0u : ((1u << (count - first)) - 1u);  // count - first < 32 here
   return keep;
 }
 
-// Exclusive scan of one 32-bit count per thread over the NC threads of a
-// warp group with one named barrier: warp totals through s_cnt (NC / 32
-// words, written again only after a later barrier of the group), then every
-// thread adds the totals of the warps before its own.
-template <int NC>
-__device__ __forceinline__ unsigned count_scan_1bar(unsigned v, unsigned *s_cnt, unsigned *total, int t, int bar) {
-  const int lane = t & 31, warp = t >> 5;
-  unsigned incl = v;
+// Aggregator warp, item by item: once every reducer warp has parked the tile,
+// count the threads' keep masks, leave each thread's output offset in the
+// tile and, with the last tile of a unit, publish the unit's kept count
+// (EARLY: the reducers have) and hand the unit to the look-back warps.  The
+// reducers scanned their counts across a barrier of their group before, 450 of
+// their 2,600 cycles per tile; now no reducer warp waits for another.  Together
+// with units of two tiles: 2^28 uint32, 3 of 8 kept, 327 -> 303 us, 2^27 int64
+// 318 -> 270, 2^24 uint32 32.7 -> 30.4.
+template <int NC, bool EARLY>
+__device__ __forceinline__ void copy_aggregator_loop(const TmaParams &p, PipeState &ps, const unsigned *keep_all,
+                                                     uint16_t *texcl_all, unsigned long long epoch_tag, int S) {
+  constexpr int K = NC / 32;
+  static_assert(K == 4 || K == 8, "one or two 16-byte rows of masks per lane");
+  const int lane = threadIdx.x & 31;
+  RingPos r;
+  unsigned held = 0;  // kept in the unit's tiles before this one
+  for (long long it = 0;; ++it, r.advance(1, S)) {
+    const int s = r.s;
+    if (aggregator_wait(p, ps, r, it) <= 0) return;
+    const long long tile = ps.tile[s];
+    // lane l: the masks of threads l K .. l K + K - 1
+    unsigned c[K], sum = 0;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += o;
-  }
-  if (lane == 31) s_cnt[warp] = incl;
-  bar_named(bar, NC);
-  unsigned before = 0, tot = 0;
+    for (int k = 0; k < K; k += 4) {
+      const uint4 m = *reinterpret_cast<const uint4 *>(keep_all + (size_t)s * NC + lane * K + k);
+      const unsigned w[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
-  for (int w = 0; w < NC / 32; ++w) {
-    const unsigned c = s_cnt[w];
-    before += w < warp ? c : 0u;
-    tot += c;
+      for (int q = 0; q < 4; ++q) {
+        c[k + q] = sum;
+        sum += (unsigned)__popc(w[q]);
+      }
+    }
+    unsigned incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    const unsigned ex = incl - sum;
+    const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+    const bool ends = unit_ends(p, tile);
+    if (lane == 0) {
+      const long long unit = tile >> p.unit_log;
+      if (!EARLY && ends && !unit_stalled(p, unit))
+        st_status(p.status + unit, held + total, epoch_tag | (unit == 0 ? kFlagPrefix : kFlagAgg));
+      ps.agg[s] = total;
+    }
+    held = ends ? 0u : held + total;
+    unsigned o[K / 2];
+#pragma unroll
+    for (int k = 0; k < K / 2; ++k) o[k] = (ex + c[2 * k]) | ((ex + c[2 * k + 1]) << 16);
+    uint16_t *dst = texcl_all + (size_t)s * NC + lane * K;
+    if constexpr (K == 8) *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    else *reinterpret_cast<uint2 *>(dst) = make_uint2(o[0], o[1]);
+    __syncwarp();
+    if (lane == 0 && ends) mbar_arrive(&ps.aggr[unit_slot(p, s)]);
   }
-  *total = tot;
-  return before + incl - v;
 }
 
 template <class T, int NC, int ITEMS, class Pred>
-__global__ void __launch_bounds__(pipe_threads(NC), 1)
+__global__ void __launch_bounds__(tmem_pipe_threads(NC), 1)
     copy_if_tmem_kernel(const __grid_constant__ CUtensorMap tin, TmaParams p, Pred pred) {
   constexpr int kTile = NC * ITEMS;
   constexpr int kEpr = 128 / (int)sizeof(T);
@@ -104,6 +137,12 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
   constexpr int kCols = ITEMS * (int)sizeof(T) / 4;
   static_assert(kCols == 16 || kCols == 32, "TMEM columns per thread");
   static_assert(NC % 128 == 0, "reducer and emitter groups cover the four TMEM lane quarters evenly");
+  // Who publishes a unit's kept count: its last reducer warp, before it waits
+  // for a slot, or the aggregator.  The first shortens every look-back but costs
+  // each reducer warp a reduction and a shared atomic per tile.  With 16
+  // elements per thread the warps have the time (2^27 int64: 270 us, by the
+  // aggregator 299), with 32 they have not (2^28 uint32: 324 and 304).
+  constexpr bool kEarly = ITEMS <= 16;
   constexpr int kSlotCols = kCols * (NC / 128);
 
   extern __shared__ char smem_raw[];
@@ -112,12 +151,12 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
   unsigned *keep_all = reinterpret_cast<unsigned *>(smem + p.texcl_base);
   uint16_t *texcl_all = reinterpret_cast<uint16_t *>(keep_all + (size_t)p.slots * NC);  // offsets < 2^16
   __shared__ __align__(8) PipeState ps;
-  __shared__ unsigned s_cnt[NC / 32];
   __shared__ int s_go[2];
+  __shared__ unsigned s_cnt[kMaxStages];  // kEarly, by unit slot: warps that counted << 24 | kept so far
 
   const int warp = threadIdx.x >> 5;
-  // aggr completes when every reducer warp has parked its part of the tile
-  tmem_pipe_init(ps, p, NC / 32, NC / 32);
+  tmem_pipe_init(ps, p, NC / 32);
+  if (threadIdx.x < kMaxStages) s_cnt[threadIdx.x] = 0;
   if (warp == 0) {
     __syncwarp();
     tmem_alloc(&ps.tmem_base, 512);
@@ -140,20 +179,11 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
     long long it = 0;
     RingPos ri, rs;
     for (;; ++it, ri.advance(1, SI), rs.advance(1, SL)) {
-      if (t == 0) {
-        int go = mbar_wait(&ps.full[ri.s], ri.ph, p.timeout_ns) ? 1 : -1;
-        if (go > 0 && ps.tile_in[ri.s] < 0) go = 0;
-        if (go > 0 && !mbar_wait(&ps.slot_free[rs.s], rs.ph ^ 1u, p.timeout_ns)) go = -1;
-        if (go < 0) record_error(p.hdr, B2P_ERR_TIMEOUT);
-        s_go[0] = go;
-      }
-      bar_named(1, NC);
-      if (s_go[0] <= 0) break;
-      (void)mbar_try(&ps.full[ri.s], ri.ph);  // completed: this thread's acquire of the TMA bytes
-      tmem_fence_after();
+      if (!warp_wait(&ps.full[ri.s], ri.ph, p)) break;
       const long long tile = ps.tile_in[ri.s];
+      if (tile < 0) break;
       char *buf = smem + (size_t)ri.s * p.stage_stride;
-      if (tile == last && ntail > 0) load_row_tail<T, NC>(p, buf, tile, kTile);
+      if (tile == last && ntail > 0) own_row_tail<T>(p, buf, tile * kTile, t * ITEMS, ITEMS);
       uint32_t w[kCols];
 #pragma unroll
       for (int k = 0; k < kCols / 4; ++k) {
@@ -169,24 +199,30 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
       // stores after it then issue without waiting
       const int count = (int)min((unsigned long long)kTile, p.n - (unsigned long long)tile * kTile);
       const unsigned keep = keep_bits<T, ITEMS>(w, pred, t * ITEMS, count);
+      const unsigned warp_kept = kEarly ? __reduce_add_sync(0xffffffffu, (unsigned)__popc(keep)) : 0u;
+      if (kEarly && (t & 31) == 0) {
+        // the unit's last warp publishes its kept count, whether or not there
+        // is a slot for the tile yet
+        const long long unit = tile >> p.unit_log, tiles = min(1ll << p.unit_log, p.ntiles - (unit << p.unit_log));
+        unsigned *cnt = &s_cnt[unit_slot(p, rs.s)];
+        const unsigned sum = atomicAdd(cnt, warp_kept + (1u << 24)) + warp_kept + (1u << 24);
+        if (sum >> 24 == (unsigned)tiles * (NC / 32)) {
+          if (!unit_stalled(p, unit))
+            st_status(p.status + unit, sum & 0xffffffu, epoch_tag | (unit == 0 ? kFlagPrefix : kFlagAgg));
+          *cnt = 0;
+        }
+      }
+      if (!warp_wait(&ps.slot_free[rs.s], rs.ph ^ 1u, p)) break;
+      tmem_fence_after();
       const uint32_t ta = tcol + (uint32_t)(rs.s * kSlotCols);
       tmem_st16(ta, w);
       if constexpr (kCols == 32) tmem_st16(ta + 16, w + 16);
-      unsigned kept32;
-      const unsigned ex = count_scan_1bar<NC>((unsigned)__popc(keep), s_cnt, &kept32, t, 1);
-      const unsigned long long tile_kept = kept32;
-      if (t == 0) {  // the kept count goes out as soon as the count scan knows it
-        if (tile != p.stall_tile)
-          st_status(p.status + tile, tile_kept, epoch_tag | (tile == 0 ? kFlagPrefix : kFlagAgg));
-        ps.tile[rs.s] = tile;
-        ps.agg[rs.s] = tile_kept;
-      }
-      texcl_all[(size_t)rs.s * NC + t] = (uint16_t)ex;
       keep_all[(size_t)rs.s * NC + t] = keep;
+      if (t == 0) ps.tile[rs.s] = tile;
       tmem_wait_st();
       tmem_fence_before();
       __syncwarp();
-      if ((t & 31) == 0) mbar_arrive(&ps.aggr[rs.s]);  // this warp's slot columns, masks and offsets
+      if ((t & 31) == 0) mbar_arrive(&ps.slot_ready[rs.s]);  // this warp's slot columns and masks
     }
     if (t == 0) *reinterpret_cast<volatile long long *>(&ps.end_item) = it;
   } else if (warp < 2 * NC / 32) {
@@ -199,13 +235,9 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
         int go = emitter_wait(p, ps, rs, it);
         if (go > 0 && !mbar_wait(&ps.out_empty[ro.s], ro.ph ^ 1u, p.timeout_ns)) go = -1;
         if (go < 0) record_error(p.hdr, B2P_ERR_TIMEOUT);
-        if (go == 0) {
-          // end the store warp and the look-back warps (waiting on items it ..
-          // it + kLookWarps - 1, each barrier completing after NC / 32 arrivals)
+        if (go == 0) {  // every item was handed on: end the store warp and the look-back warps
           mbar_arrive(&ps.emitted[ro.s]);
-          RingPos r = rs;
-          for (int j = 0; j < kLookWarps; ++j, r.advance(1, SL))
-            for (int k = 0; k < NC / 32; ++k) mbar_arrive(&ps.aggr[r.s]);
+          end_lookback_units(p, ps, rs, it, SL);
         }
         s_go[1] = go;
       }
@@ -234,31 +266,28 @@ __global__ void __launch_bounds__(pipe_threads(NC), 1)
       const unsigned phase = (unsigned)(g0 & 15u);
       if (!broken) {
         T *ob = reinterpret_cast<T *>(obuf + phase) + o;  // phase is a multiple of sizeof(T)
-        unsigned pos = 0;
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
-          const unsigned b = (keep >> j) & 1u;
-          if (b) {
-            T v;
-            memcpy(&v, w + j * (int)(sizeof(T) / 4), sizeof(T));
-            ob[pos] = v;
-          }
-          pos += b;
+          T v;
+          memcpy(&v, w + j * (int)(sizeof(T) / 4), sizeof(T));
+          if (keep & (1u << j)) *ob++ = v;
         }
       }
       fence_async_smem();
-      bar_named(2, NC);  // the output stage is packed
-      if (t == 0 && tile == last && p.num_copied) *p.num_copied = carry + kept_total;
       if (t == 0) {
+        if (tile == last && p.num_copied) *p.num_copied = carry + kept_total;
         ps.out_carry[ro.s] = carry;
         ps.out_count[ro.s] = kept_total;
-        mbar_arrive(&ps.emitted[ro.s]);
       }
+      bar_named(2, NC);
+      if (t == 0) mbar_arrive(&ps.emitted[ro.s]);
     }
   } else if (warp < 2 * NC / 32 + kLookWarps) {
-    lookback_loop<CountOps>(p, ps, warp - 2 * NC / 32, 0ull, epoch_tag, SL);
+    lookback_unit_loop<CountOps>(p, ps, warp - 2 * NC / 32, 0ull, epoch_tag, SL);
   } else if (warp == 2 * NC / 32 + kLookWarps) {
     if ((threadIdx.x & 31) == 0) producer_loop(&tin, p, ps, smem, kRows, kBox, ps.tile_in);
+  } else if (warp == 2 * NC / 32 + kLookWarps + 2) {
+    copy_aggregator_loop<NC, kEarly>(p, ps, keep_all, texcl_all, epoch_tag, SL);
   } else {
     // ---------------------------------------------------------- store warp
     if ((threadIdx.x & 31) == 0) {
@@ -322,7 +351,10 @@ inline bool copy_tmem_layout(TmaParams &p, size_t es, int block, int items) {
   const size_t side = ((size_t)slots * block * 6 + 1023) & ~size_t(1023);
   const int so = kCopyOutStages;
   if (so * out_b + side + 2 * in_b > kSmemBudget) return false;
-  const int si = (int)std::min<size_t>(kMaxStages, (kSmemBudget - so * out_b - side) / in_b);
+  // A reducer warp counts its part of a tile before the tile's slot is free.
+  // It holds an input stage then, so with two stages fewer than slots every
+  // warp is done with the tiles that used the unit's counter before.
+  const int si = (int)std::min<size_t>(slots - 2, (kSmemBudget - so * out_b - side) / in_b);
   p.stages = si;
   p.stage_stride = (unsigned)in_b;
   p.slots = slots;
@@ -358,14 +390,16 @@ int launch_copy_tmem_shape(TmaParams &p, const CUtensorMap &tin, const Pred &pre
       int nb = 0;
       bool ok = cudaFuncSetAttribute((const void *)kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
                 cudaSuccess;
-      ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)kfn, pipe_threads(NC), smem) ==
+      ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)kfn, tmem_pipe_threads(NC), smem) ==
                      cudaSuccess && nb >= 1;
       if (!ok) cudaGetLastError();
       st_once.store(ok ? 1 : 2);
     }
     if (st_once.load() != 1) return B2P_ERR_UNSUPPORTED;
+    TmaParams q = p;
+    q.unit_log = look_back_unit_log(p, sm_count);
     const int grid = (int)std::min<long long>(p.ntiles, (long long)sm_count);
-    kfn<<<grid, pipe_threads(NC), smem, st>>>(tin, p, pred);
+    kfn<<<grid, tmem_pipe_threads(NC), smem, st>>>(tin, q, pred);
     return cudaGetLastError() == cudaSuccess ? B2P_OK : B2P_ERR_CUDA;
   }
 }

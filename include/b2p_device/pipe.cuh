@@ -49,12 +49,18 @@ constexpr int kScanOutStages = 2;
 constexpr int kTmemStoresInFlight = 1;
 constexpr int kScanMaxInStages = kMaxStages;
 
-// Threads of a pipelined block with NC reducer and NC emitter threads.
+// Threads of a pipelined block with NC reducer and NC emitter threads, and of
+// one that has an aggregator warp too.
 constexpr int pipe_threads(int nc) { return 2 * nc + 32 * kLookWarps + 64; }
+constexpr int tmem_pipe_threads(int nc) { return pipe_threads(nc) + 32; }
 
 struct TmaParams {
   unsigned long long n;
   long long ntiles;
+  // log2 of the tiles per look-back unit (a divisor of slots).  A block takes
+  // the tiles of a unit one after the other, publishes one aggregate for them
+  // and looks back once.
+  int unit_log = 0;
   long long rows_full;            // complete 128-byte input rows (the input tensor map's extent)
   unsigned long long tail_begin;  // first element past the complete input rows
   long long rows_full_out;        // complete 128-byte output rows (scans)
@@ -94,6 +100,15 @@ struct TmaParams {
   unsigned rend_base;  // ... of the per-slot entering-segment ends (reduce)
   unsigned rec_base;   // ... of the per-stage tile records
 };
+
+// Host: log2 of the tiles per look-back unit of a TMEM-staged launch.  Two tiles
+// once every SM has three (2^21 uint32, 1.7 per SM: copy_if 14.4 us with two,
+// 13.5 with one; 6 x 2^20: 18.4 and 19.9), one below, where a unit of two
+// leaves SMs without work.  Four tiles per unit keep half a block's slots
+// waiting for one look-back: 2^28 floats 371 us against 357 with two.
+inline int look_back_unit_log(const TmaParams &p, int sm_count) {
+  return p.slots % 2 == 0 && p.slots >= 2 * kLookWarps && p.ntiles >= 3ll * sm_count ? 1 : 0;
+}
 
 // Per-tile record of the segmented kernel: 64 ints = 256 bytes.
 constexpr int kSegRecInts = 64;
@@ -331,12 +346,13 @@ __device__ __forceinline__ void pipe_init(PipeState &ps, const TmaParams &p) {
   }
 }
 
-// Producer (one thread): each tile's complete rows into the next free stage
+// Producer (one thread): dynamic unit ids in order; each tile's complete rows
+// into the next free stage
 // in boxes of `box` rows, and, when `rec_g` is given, the tile's
 // `rec_bytes`-byte record (rec_g + tile * rec_bytes) into rec_s + stage *
 // rec_bytes on the same barrier.  A tile wholly past the complete rows
 // completes its stage without a row copy.  Tile id -1 ends the reducers.
-// The next tile id is fetched while the current one is issued, so the
+// The next unit id is fetched while the current one is issued, so the
 // counter's round trip overlaps the stage wait; ids stay in order per
 // block, and every id a block holds is loaded as soon as it has a stage (a
 // block only ever waits for tiles of lower ids, so every wait ends).
@@ -348,7 +364,8 @@ __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaP
   prefetch_tensormap(tin);
   const unsigned long long pol = l2_policy_stream();
   const int S = p.stages;
-  long long next = (long long)atomicAdd(&p.hdr->tile_ctr, 1ull);
+  long long unit = (long long)atomicAdd(&p.hdr->tile_ctr, 1ull), next = 0;
+  int part = 0;
   for (RingPos r;; r.advance(1, S)) {
     const int s = r.s;
     if (!mbar_wait(&ps.empty[s], r.ph ^ 1u, p.timeout_ns)) {
@@ -357,14 +374,18 @@ __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaP
       mbar_arrive(&ps.full[s]);
       return;
     }
-    const long long tile = next;
+    const long long tile = (unit << p.unit_log) + part;
     if (tile >= p.ntiles) {
       tiles[s] = -1;
       mbar_arrive(&ps.full[s]);
       if (--end_markers > 0) continue;
       return;
     }
-    next = (long long)atomicAdd(&p.hdr->tile_ctr, 1ull);
+    if (part == 0) next = (long long)atomicAdd(&p.hdr->tile_ctr, 1ull);
+    if (++part >> p.unit_log) {
+      part = 0;
+      unit = next;
+    }
     tiles[s] = tile;
     const long long r0 = tile * rows;
     const long long rows_in = min((long long)rows, p.rows_full - r0);
@@ -380,6 +401,68 @@ __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaP
       if (extra) bulk_load(rec_s + (size_t)s * rec_bytes, rec_g + (size_t)tile * rec_bytes, rec_bytes, &ps.full[s], pol);
     }
   }
+}
+
+// mbar_wait() by a whole warp: every lane waits (and so acquires what the
+// barrier's arrivals and copies published); one outcome for the warp.
+__device__ __forceinline__ bool warp_wait(uint64_t *b, unsigned parity, const TmaParams &p) {
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(b, parity, p.timeout_ns));
+  if (!ok && (threadIdx.x & 31) == 0) record_error(p.hdr, B2P_ERR_TIMEOUT);
+  return ok;
+}
+
+// One thread's elements [first, first + count) of the last tile that lie past
+// the complete rows, from global memory into the thread's own part of the
+// stage.
+template <class T>
+__device__ __forceinline__ void own_row_tail(const TmaParams &p, char *buf, long long tile0, int first, int count) {
+  for (int j = first; j < first + count; ++j) {
+    const unsigned long long i = (unsigned long long)(tile0 + j);
+    if (i >= p.tail_begin && i < p.n) *smem_elem_ptr<T>(buf, j) = reinterpret_cast<const T *>(p.in)[i];
+  }
+}
+
+// Aggregator warp, item `it` in slot s: wait until every reducer warp has
+// parked the tile (slot_ready).  1 = parked, 0 = the block's items are
+// exhausted, -1 = timeout; the same for the whole warp.
+__device__ __forceinline__ int aggregator_wait(const TmaParams &p, PipeState &ps, const RingPos &r, long long it) {
+  int go = 0;
+  if ((threadIdx.x & 31) == 0) {
+    uint64_t t0 = 0;
+    for (unsigned k = 0;; ++k) {
+      if (mbar_try_hint(&ps.slot_ready[r.s], r.ph, 2000)) {
+        go = 1;
+        break;
+      }
+      if (it >= *reinterpret_cast<volatile long long *>(&ps.end_item)) break;
+      if ((k & 7) == 7) {
+        const uint64_t now = globaltimer_ns();
+        if (t0 == 0) {
+          t0 = now;
+        } else if (now - t0 > p.timeout_ns) {
+          record_error(p.hdr, B2P_ERR_TIMEOUT);
+          go = -1;
+          break;
+        }
+      }
+    }
+  }
+  go = __shfl_sync(0xffffffffu, go, 0);
+  if (go > 0) (void)mbar_try(&ps.slot_ready[r.s], r.ph);  // completed: this lane's acquire of the parked words
+  return go;
+}
+
+// The time-out test's hook: the unit of this tile never publishes.
+__device__ __forceinline__ bool unit_stalled(const TmaParams &p, long long unit) {
+  return p.stall_tile >= 0 && p.stall_tile >> p.unit_log == unit;
+}
+
+// First slot of the unit in slot s.
+__device__ __forceinline__ int unit_slot(const TmaParams &p, int s) { return s >> p.unit_log << p.unit_log; }
+
+// Whether a tile is the last of its unit.
+__device__ __forceinline__ bool unit_ends(const TmaParams &p, long long tile) {
+  return (((unsigned)tile + 1) & ((1u << p.unit_log) - 1)) == 0 || tile + 1 == p.ntiles;
 }
 
 // Look-back warp wi of kLookWarps: items wi, wi + kLookWarps, ... in stage
@@ -422,6 +505,55 @@ __device__ __forceinline__ void lookback_loop(const TmaParams &p, PipeState &ps,
   }
 }
 
+// The same by units of tiles (TMEM-staged kernels): the aggregator
+// arrives on aggr of a unit's first slot once all its tiles are parked and its
+// aggregate is published; one look-back gives the carries of all of them.
+//
+// A look-back takes about 2.6 us while DRAM runs at full rate: a poll of 128
+// words is a slow round trip, and every tile in flight on the GPU, 8 per SM,
+// lies between a tile and the nearest published prefix.  Two warps then carry
+// 0.77 tiles per us and SM, where copy_if needs 0.9 and a bf16 scan 0.85; more
+// warps only slow the polls down (2^28 floats: 385 us with two, 411 with
+// four).  Two tiles per unit halve both the look-backs and the distance: 2^28
+// uint32 371 -> 354 us, 2^27 int64 377 -> 353.
+template <class Ops>
+__device__ __forceinline__ void lookback_unit_loop(const TmaParams &p, PipeState &ps, int wi,
+                                                   unsigned long long init_bits, unsigned long long epoch_tag, int S) {
+  using Pub = typename Ops::Pub;
+  const int lane = threadIdx.x & 31, U = 1 << p.unit_log;
+  RingPos r;
+  r.advance(wi * U, S);
+  for (long long k = wi;; k += kLookWarps, r.advance(kLookWarps * U, S)) {
+    const int s = r.s;
+    if (!warp_wait(&ps.aggr[s], r.ph, p)) return;
+    if (k * U >= *reinterpret_cast<volatile long long *>(&ps.end_item)) return;
+    const long long tile = ps.tile[s], unit = tile >> p.unit_log;
+    const int nt = (int)min((long long)U, p.ntiles - tile);
+    Pub carry = Ops::unpack(init_bits);
+    if (unit > 0) {
+      bool err;
+      // unit 0's prefix includes init, so the look-back result already does
+      carry = lookback<Ops, false>(p.status, unit, epoch_tag, p.timeout_ns, err);
+      if (lane == 0) {
+        if (err) record_error(p.hdr, B2P_ERR_TIMEOUT);
+        Pub sum = Ops::unpack(ps.agg[s]);
+        for (int j = 1; j < nt; ++j) sum = Ops::combine(sum, Ops::unpack(ps.agg[s + j]));
+        if (!unit_stalled(p, unit))
+          st_status(p.status + unit, Ops::pack(Ops::combine(carry, sum)),
+                    epoch_tag | kFlagPrefix | (err ? kFlagError : 0));
+      }
+    }
+    if (lane == 0) {
+      for (int j = 0; j < nt; ++j) {
+        ps.carry[s + j] = Ops::pack(carry);
+        mbar_arrive(&ps.cready[s + j]);
+        if (j + 1 < nt) carry = Ops::combine(carry, Ops::unpack(ps.agg[s + j]));
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // Emitter group: wait for item `it`'s carry, or learn that the block's items
 // are exhausted (the reducers publish the count when they meet the end).
 // Returns 1 = carry ready, 0 = no more items, -1 = timeout.
@@ -446,6 +578,15 @@ __device__ __forceinline__ int emitter_wait(const TmaParams &p, PipeState &ps, c
 __device__ __forceinline__ void emitters_finish(const TmaParams &p, PipeState &ps, RingPos r) {
   mbar_arrive(&ps.emitted[r.s]);
   for (int j = 0; j < kLookWarps; ++j, r.advance(1, p.stages)) mbar_arrive(&ps.aggr[r.s]);
+}
+
+// One thread, after `it` items, each handed on by the look-back warps: end the
+// look-back warps of lookback_unit_loop(), which wait on the first slots of the
+// next kLookWarps units (r: the position of item `it`).
+__device__ __forceinline__ void end_lookback_units(const TmaParams &p, PipeState &ps, RingPos r, long long it, int S) {
+  const int U = 1 << p.unit_log, over = (int)it & (U - 1);
+  if (over) r.advance(U - over, S);  // a last unit of fewer tiles
+  for (int j = 0; j < kLookWarps; ++j, r.advance(U, S)) mbar_arrive(&ps.aggr[r.s]);
 }
 
 // Store warp: stages whose bulk stores were committed but may still read
@@ -498,15 +639,14 @@ constexpr int tmem_cols() {
 // Thread 0: barriers of the three rings (input stages, TMEM slots, output
 // stages) and the launch epoch.  Reducer and emitter warps arrive one by one
 // on the barriers that hand back input stages and slots.
-__device__ __forceinline__ void tmem_pipe_init(PipeState &ps, const TmaParams &p, unsigned group_warps,
-                                               unsigned aggr_count = 1) {
+__device__ __forceinline__ void tmem_pipe_init(PipeState &ps, const TmaParams &p, unsigned group_warps) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.stages; ++i) {
       mbar_init(&ps.full[i], 1);
       mbar_init(&ps.empty[i], group_warps);
     }
     for (int i = 0; i < p.slots; ++i) {
-      mbar_init(&ps.aggr[i], aggr_count);
+      mbar_init(&ps.aggr[i], 1);
       mbar_init(&ps.cready[i], 1);
       mbar_init(&ps.slot_free[i], group_warps);
       mbar_init(&ps.slot_ready[i], group_warps);

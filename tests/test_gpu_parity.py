@@ -533,3 +533,62 @@ def test_scan_and_copy_if_at_the_tile_rules(dev, code):
             ref = torch.cumsum(x.to(torch.float64), 0)
             got = C.inclusive_scan(x).to(torch.float64)
             assert ((got - ref).abs() <= 1e-6 * ref.abs() + 1e-30).all(), n
+
+
+@pytest.mark.parametrize("code", [C.U32, C.I64, C.F32, C.BF16])
+def test_pipelined_look_back_units(dev, code):
+    """Tile counts around the rule for two tiles per look-back unit (three per
+    SM), with a last unit of one tile and ragged last tiles: integer scans and
+    copy_if (few, some and all kept) exact, float scans within 1e-6 of FP64."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(code)
+    for items in (16, 32):
+        if code == C.I64 and items == 32:
+            continue
+        cfg = 16 + 4 + (2 if items == 16 else 3)
+        tile = 256 * items
+        for n in [t * tile + d for t in (3 * sms - 1, 3 * sms, 3 * sms + 1) for d in (-1, 0, 1, 5)]:
+            if code in (C.U32, C.I64):
+                x = torch.randint(0, 1 << 20, (n,), generator=g, device="cuda")
+                ref = torch.cumsum(x, 0)
+                y = x if code == C.I64 else x.to(torch.uint32)
+                got = C.inclusive_scan(y, config=cfg).to(torch.int64)
+                assert torch.equal(got, ref if code == C.I64 else ref & 0xFFFFFFFF), (items, n)
+                for rhs in (0, 1, 3, 8):
+                    out, cnt = C.copy_if(y, 7, C.CMP_LT, rhs, config=cfg)
+                    keep = x[(x & 7) < rhs]
+                    k = int(cnt.item())
+                    assert k == keep.numel() and torch.equal(out[:k].to(torch.int64), keep), (items, n, rhs)
+            else:
+                x = torch.rand(n, generator=g, device="cuda").to(torch.float32 if code == C.F32 else torch.bfloat16)
+                ref = torch.cumsum(x.to(torch.float64), 0)
+                got = C.inclusive_scan(x, config=cfg).to(torch.float64)
+                assert ((got - ref).abs() <= 1e-6 * ref).all(), (items, n)
+
+
+@pytest.mark.parametrize("code", [C.F32, C.BF16])
+def test_pipelined_scan_special_values(dev, code):
+    """Denormals and signed zeros scan like other values; from an infinity or a
+    NaN on, and only there, the outputs are not finite."""
+    n = 6 << 20
+    dt = torch.float32 if code == C.F32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(code)
+    bits = torch.randint(0, 1 << (23 if code == C.F32 else 7), (n,), generator=g, device="cuda")
+    tiny = bits.to(torch.int32 if code == C.F32 else torch.int16).view(dt)
+    ref = torch.cumsum(tiny.to(torch.float64), 0)
+    got = C.inclusive_scan(tiny).to(torch.float64)
+    # one fp32 rounding: relative, or half a denormal step of 2^-149
+    assert ((got - ref).abs() <= 1e-6 * ref + 2.0**-149).all()
+    assert (C.inclusive_scan(torch.full((n,), -0.0, device="cuda", dtype=dt)) == 0).all()
+    x = torch.rand(n, generator=g, device="cuda").to(dt)
+    for at, value in ((n // 2 + 3, float("inf")), (n // 3, float("-inf")), (n - 2, float("nan"))):
+        y = x.clone()
+        y[at] = value
+        ref = torch.cumsum(y.to(torch.float64), 0)
+        for got, start in ((C.inclusive_scan(y), at), (C.exclusive_scan(y, 0.0), at + 1)):
+            # (the double-float carry of an infinity is (inf, NaN): NaN in later tiles)
+            assert not torch.isfinite(got[start:]).any()
+            assert got[start].item() == value or value != value
+            assert torch.isfinite(got[:start]).all()
+        inc = C.inclusive_scan(y)[:at].to(torch.float64)
+        assert ((inc - ref[:at]).abs() <= 1e-6 * ref[:at]).all()
