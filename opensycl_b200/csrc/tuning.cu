@@ -53,11 +53,13 @@ int heuristic_config(int prim, int dtype, size_t n, int64_t nseg) {
   case B2P_PRIM_SCAN:
   case B2P_PRIM_COPY_IF: {
     // The pipelined (TMA) kernel once its blocks have several tiles each: a scan
-    // beyond 16 MiB (2^22 int32: 15.5 us against 14.0 us of the look-back
-    // kernel; 2^23: 37 against 50), copy_if from 8 MiB of input on (2^21
-    // uint32: 11.2 against 14.0).
+    // beyond 16 MiB (2^22 int32: 13.8 us against 13.0 us of the look-back
+    // kernel; 5 x 2^20: 15.0 against 17.4), copy_if beyond 13 MiB of uint32
+    // (3 x 2^20: 15.2 against 13.3; 2^22: 15.8 against 20.3) and 16 MiB of int64
+    // (2^21: 15.8 against 15.4; 3 x 2^20: 17.5 against 21.3).
     const bool scan = prim == B2P_PRIM_SCAN;
-    if (scan ? n * acc_size(dtype) > (16u << 20) : bytes >= (8u << 20)) return cfg(1, 256, es == 8 ? 16 : 32);
+    if (scan ? n * acc_size(dtype) > (16u << 20) : bytes > ((es == 8 ? 16u : 13u) << 20))
+      return cfg(1, 256, es == 8 ? 16 : 32);
     // Below, one look-back tile per block: the smallest tile that still leaves
     // at most about one tile per SM, because the time is the latency of one
     // tile and the look-back over the others (2^16 int32: 5.5 us with 2048
@@ -66,7 +68,7 @@ int heuristic_config(int prim, int dtype, size_t n, int64_t nseg) {
     if (n <= (1u << 18)) return es == 2 ? cfg(0, 256, 8) : cfg(0, 512, 4);
     if (n <= (1u << 19)) return es == 4 ? cfg(0, 1024, 4) : cfg(0, 512, 8);
     if (scan && es == 8) return cfg(0, 256, 16);
-    if (n <= (1u << 20)) return cfg(0, 1024, 8);
+    if (n <= (1u << 20) || es == 8) return cfg(0, 1024, 8);
     return n <= (1u << 21) ? cfg(0, 512, 16) : cfg(0, 256, 32);
   }
   case B2P_PRIM_HISTOGRAM:

@@ -517,7 +517,7 @@ def test_scan_and_copy_if_at_the_tile_rules(dev, code):
     against a mask, integers exact, floats within 1e-6."""
     g = torch.Generator(device="cuda").manual_seed(code)
     for n in (1, 2048, 2049, 1 << 18, (1 << 18) + 1, 1 << 19, (1 << 19) + 1, 1 << 20, (1 << 20) + 1, 1 << 21,
-              (1 << 21) + 1, 1 << 22, (1 << 22) + 1):
+              (1 << 21) + 1, 13 << 18, (13 << 18) + 1, 1 << 22, (1 << 22) + 1):
         if code in (C.I32, C.I64):
             x = torch.randint(0, 1 << 20, (n,), generator=g, device="cuda")
             x = x.to(torch.int32 if code == C.I32 else torch.int64)
