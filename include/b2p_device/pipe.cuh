@@ -636,6 +636,126 @@ constexpr int tmem_cols() {
   return ITEMS * (int)sizeof(typename P::Out) / 4;
 }
 
+// FP64 value of a float (bf16: of its two halves) times 2^-896, by its bits:
+// the float's exponent and mantissa fields moved into the double's, exact for
+// every finite value, zeros and denormals too.  A conversion instruction runs
+// at 16 lanes per clock and SM, and the rounding of the outputs needs one per
+// element as well; the integer operations run at 64, and the factor costs
+// nothing: the running sum takes the value by an fma with 2^896, the same
+// rounding.  2^28 floats 372 -> 358 us, 5 x 10^7 bf16 74.0 -> 68.3.
+__device__ __forceinline__ double scaled_f64(unsigned u) {
+  return __hiloint2double((int)(((unsigned)((int)u >> 3)) & 0x8fffffffu), (int)(u << 29));
+}
+__device__ __forceinline__ double scaled_bf16_hi(unsigned w) {
+  return __hiloint2double((int)(((unsigned)((int)w >> 3)) & 0x8fffe000u), 0);
+}
+__device__ __forceinline__ double scaled_bf16_lo(unsigned w) {
+  return __hiloint2double((int)(((unsigned)((int)(w << 16) >> 3)) & 0x8fffe000u), 0);
+}
+constexpr double kUnscale = 0x1p896;
+
+// The compensated pass below with converted values, out of line so that its
+// registers are not the common path's.
+template <class P, int ITEMS, bool INCL>
+__device__ __noinline__ double converted_runs(const char *inbuf, uint32_t *w, int t) {
+  using In = typename P::In;
+  constexpr int IPV = 16 / (int)sizeof(In);
+  double rd = 0.0;
+  for (int j = 0; j < ITEMS; ++j) {
+    const In e = reinterpret_cast<const In *>(inbuf + swz(t * (ITEMS / IPV) + j / IPV) * 16)[j % IPV];
+    const double x = (double)P::lift_f(e);
+    w[j] = __float_as_uint((float)(INCL ? rd + x : rd));
+    rd += x;
+  }
+  return rd;
+}
+
+// Reducer pass: the thread's ITEMS elements from the landed stage, their
+// running values from the identity (inclusive: after adding the element,
+// exclusive: before) as 32-bit words for TMEM, and the thread total.
+// Compensated sums (fp32 / bf16) run in FP64: the thread's values are exact
+// in FP64 and their sum far inside its precision, each parked word is one
+// rounding of the running value, and the total leaves as the double-float
+// (hi, lo) split of the FP64 sum.  A thread that holds an infinity or a NaN
+// (x * 0 is not 0) repeats its pass with converted values.
+template <class P, int ITEMS, bool INCL>
+__device__ __forceinline__ typename P::Acc tmem_runs(const char *inbuf, uint32_t *w, int t) {
+  using In = typename P::In;
+  using Out = typename P::Out;
+  constexpr int IPV = 16 / (int)sizeof(In), VPT = ITEMS / IPV, WPO = (int)sizeof(Out) / 4;
+  if constexpr (P::kCompensated) {
+    double rd = 0.0;
+    auto put = [&](int j) { w[j] = __float_as_uint((float)rd); };
+    bool finite;
+    if constexpr (sizeof(In) == 4) {
+      float zero = 0.f;
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(inbuf + swz(t * VPT + k) * 16);
+        const unsigned e[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          zero = __fmaf_rn(__uint_as_float(e[q]), 0.f, zero);
+          if constexpr (!INCL) put(k * IPV + q);
+          rd = __fma_rn(scaled_f64(e[q]), kUnscale, rd);
+          if constexpr (INCL) put(k * IPV + q);
+        }
+      }
+      finite = zero == 0.f;
+    } else {
+      __nv_bfloat162 zero = __float2bfloat162_rn(0.f);
+      const __nv_bfloat162 z = zero;
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const uint4 u = *reinterpret_cast<const uint4 *>(inbuf + swz(t * VPT + k) * 16);
+        const unsigned e[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          __nv_bfloat162 pair;
+          memcpy(&pair, &e[q], 4);
+          zero = __hfma2(pair, z, zero);
+          if constexpr (!INCL) put(k * IPV + 2 * q);
+          rd = __fma_rn(scaled_bf16_lo(e[q]), kUnscale, rd);
+          put(k * IPV + 2 * q + (INCL ? 0 : 1));
+          rd = __fma_rn(scaled_bf16_hi(e[q]), kUnscale, rd);
+          if constexpr (INCL) put(k * IPV + 2 * q + 1);
+        }
+      }
+      unsigned zb;
+      memcpy(&zb, &zero, 4);
+      finite = (zb & 0x7fff7fffu) == 0;
+    }
+    if (!finite) {
+      uint32_t c[ITEMS];
+      rd = converted_runs<P, ITEMS, INCL>(inbuf, c, t);
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) w[j] = c[j];
+    }
+    const float h = (float)rd;
+    return typename P::Acc{h, (float)(rd - (double)h)};
+  } else {
+    typename P::Acc run = P::identity();
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const uint4 u = *reinterpret_cast<const uint4 *>(inbuf + swz(t * VPT + k) * 16);
+      const In *e = reinterpret_cast<const In *>(&u);
+#pragma unroll
+      for (int q = 0; q < IPV; ++q) {
+        Out o;
+        if constexpr (INCL) {
+          P::add(run, e[q]);
+          o = P::finalize(run);
+        } else {
+          o = P::finalize(run);
+          P::add(run, e[q]);
+        }
+        memcpy(w + (k * IPV + q) * WPO, &o, sizeof(Out));
+      }
+    }
+    return run;
+  }
+}
+
 // Thread 0: barriers of the three rings (input stages, TMEM slots, output
 // stages) and the launch epoch.  Reducer and emitter warps arrive one by one
 // on the barriers that hand back input stages and slots.

@@ -167,3 +167,31 @@ def test_segmented_offsets_checked_on_device(dev, nseg):
     bad[0] = -1
     with pytest.raises(C.B2PError):
         C.segmented_reduce(xd, torch.from_numpy(bad).cuda(), "sum")
+
+
+@pytest.mark.parametrize("code", [C.F32, C.BF16])
+@pytest.mark.parametrize("inclusive", [True, False])
+def test_segmented_scan_special_values(dev, code, inclusive):
+    """Long and short segments with denormals, and an infinity or a NaN in some
+    of them: those segments are not finite from that element on, every other
+    output is within 1e-6 of FP64 sums."""
+    n, dt = 3 * 8192 * 40 + 777, torch.float32 if code == C.F32 else torch.bfloat16
+    rng = np.random.default_rng(int(code) + inclusive)
+    cuts = np.unique(np.concatenate([rng.integers(0, n, 60), rng.integers(n // 2, n // 2 + 4000, 200), [0, n]]))
+    x = torch.from_numpy(rng.random(n).astype(np.float32)).to(dt)
+    x[1000:9000] = torch.finfo(dt).tiny / 4
+    seg = np.searchsorted(cuts, np.arange(n), side="right") - 1
+    bad_at = {int(seg[i]): int(i) for i in (n // 3, n // 2 + 1500, n - 5)}
+    for (s, i), v in zip(sorted(bad_at.items()), (float("inf"), float("-inf"), float("nan"))):
+        x[i] = v
+    xd = x.to(dev)
+    offsets = torch.from_numpy(cuts.astype(np.int64)).to(dev)
+    got = C.segmented_scan(xd, offsets, inclusive=inclusive, init=None if inclusive else 0.0).double().cpu().numpy()
+    xs = x.double().numpy()
+    for s in range(len(cuts) - 1):
+        a, b = cuts[s], cuts[s + 1]
+        fin = bad_at[s] + (0 if inclusive else 1) if s in bad_at else b
+        ref = np.cumsum(xs[a:b]) if inclusive else np.concatenate([[0.0], np.cumsum(xs[a:b])[:-1]])
+        k = fin - a
+        assert (np.abs(got[a:fin] - ref[:k]) <= 1e-6 * np.abs(ref[:k]) + 2.0**-149).all(), s
+        assert not np.isfinite(got[fin:b]).any(), s
