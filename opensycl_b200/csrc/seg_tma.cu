@@ -705,7 +705,11 @@ bool seg_layout(TmaParams &p, int block, int items) {
     // stages leave four slots at 32 KiB tiles, three all eight (2^27 int64,
     // 10000 segments 452 -> 384 us, 20 segments 494 -> 367).
     if (fixed + 3 * (in_b + rec_b) > kSmemBudget) continue;
-    const int si = (int)std::min<size_t>(kScanMaxInStages, (kSmemBudget - fixed) / (in_b + rec_b));
+    int si = (int)std::min<size_t>(kScanMaxInStages, (kSmemBudget - fixed) / (in_b + rec_b));
+    // Each reducer group has to see every phase of the stages it waits on (a
+    // barrier only tells two phases apart), so a stage belongs to one group: a
+    // multiple of the groups.
+    si -= si % seg_groups(block, REDUCE);
     p.stages = si;
     p.stage_stride = (unsigned)in_b;
     p.slots = slots;

@@ -195,3 +195,17 @@ def test_segmented_scan_special_values(dev, code, inclusive):
         k = fin - a
         assert (np.abs(got[a:fin] - ref[:k]) <= 1e-6 * np.abs(ref[:k]) + 2.0**-149).all(), s
         assert not np.isfinite(got[fin:b]).any(), s
+
+
+def test_segmented_reduce_sixteen_stage_tiles(dev):
+    """bf16 at 256 x 16 (8 KiB tiles, the shape with the most input stages):
+    many tiles per reducer group, sums within 1e-6 of FP64."""
+    n, nseg, cfg = (1 << 24) + 321, 900, 16 + 4 + 2
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.rand(n, generator=g, device="cuda").to(torch.bfloat16)
+    cuts = torch.sort(torch.randint(0, n, (nseg - 1,), generator=g, device="cuda")).values
+    offsets = torch.cat([cuts.new_zeros(1), cuts, cuts.new_full((1,), n)])
+    total = torch.cat([cuts.new_zeros(1, dtype=torch.float64), torch.cumsum(x.double(), 0)])
+    ref = total[offsets[1:]] - total[offsets[:-1]]
+    got = C.segmented_reduce(x, offsets, config=cfg).double()
+    assert ((got - ref).abs() <= 1e-6 * ref + 1e-6).all()
