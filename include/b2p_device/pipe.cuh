@@ -357,6 +357,10 @@ __device__ __forceinline__ void pipe_init(PipeState &ps, const TmaParams &p) {
 // block, and every id a block holds is loaded as soon as it has a stage (a
 // block only ever waits for tiles of lower ids, so every wait ends).
 // `end_markers` consumer groups take items in turn; each gets an end marker.
+// UNITS: look-back units may hold several tiles (p.unit_log).  A segmented
+// reduce, whose producer is the slow side, goes without: 2^28 int64 350 us
+// against 383.
+template <bool UNITS = true>
 __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaParams &p, PipeState &ps,
                                               char *smem, int rows, int box, long long *tiles,
                                               const char *rec_g = nullptr, char *rec_s = nullptr,
@@ -374,7 +378,11 @@ __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaP
       mbar_arrive(&ps.full[s]);
       return;
     }
-    const long long tile = (unit << p.unit_log) + part;
+    if (!UNITS ? part != 0 : part >> p.unit_log) {  // (here: a copy right after the atomic would wait for it)
+      part = 0;
+      unit = next;
+    }
+    const long long tile = UNITS ? (unit << p.unit_log) + part : unit;
     if (tile >= p.ntiles) {
       tiles[s] = -1;
       mbar_arrive(&ps.full[s]);
@@ -382,10 +390,7 @@ __device__ __forceinline__ void producer_loop(const CUtensorMap *tin, const TmaP
       return;
     }
     if (part == 0) next = (long long)atomicAdd(&p.hdr->tile_ctr, 1ull);
-    if (++part >> p.unit_log) {
-      part = 0;
-      unit = next;
-    }
+    ++part;
     tiles[s] = tile;
     const long long r0 = tile * rows;
     const long long rows_in = min((long long)rows, p.rows_full - r0);

@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(seg_threads(NC, REDUCE), 1)
     }
   } else if (warp == kWorkWarps + kLookWarps) {
     if ((threadIdx.x & 31) == 0)
-      producer_loop(&tin, p, ps, smem, kRows, kBox, ps.tile_in, reinterpret_cast<const char *>(p.seg_rec),
+      producer_loop<false>(&tin, p, ps, smem, kRows, kBox, ps.tile_in, reinterpret_cast<const char *>(p.seg_rec),
                     smem + p.rec_base, (unsigned)(kSegRecInts * sizeof(int)), kGroups);
   } else if constexpr (!REDUCE) {
     // ---------------------------------------------------------- store warp
