@@ -502,11 +502,26 @@ __device__ __forceinline__ void lookback_loop(const TmaParams &p, PipeState &ps,
                     epoch_tag | kFlagPrefix | (err ? kFlagError : 0));
       }
     }
+    __syncwarp();  // every lane has read the slot
     if (lane == 0) {
       ps.carry[s] = Ops::pack(carry);
       mbar_arrive(&ps.cready[s]);
     }
     __syncwarp();
+  }
+}
+
+// The carries of a unit's nt tiles, the first one's given: give(j, c) hands
+// tile j's slot on with carry c.  From then on emitters may free the slot,
+// reducers park a later tile in it and the aggregator write that tile's
+// aggregate, so agg(j) is read before.
+#pragma nv_exec_check_disable
+template <class Ops, class Agg, class Give>
+__host__ __device__ __forceinline__ void hand_on_carries(typename Ops::Pub carry, int nt, Agg agg, Give give) {
+  for (int j = 0; j < nt; ++j) {
+    const typename Ops::Pub next = j + 1 < nt ? Ops::combine(carry, agg(j)) : carry;
+    give(j, carry);
+    carry = next;
   }
 }
 
@@ -548,13 +563,14 @@ __device__ __forceinline__ void lookback_unit_loop(const TmaParams &p, PipeState
                     epoch_tag | kFlagPrefix | (err ? kFlagError : 0));
       }
     }
-    if (lane == 0) {
-      for (int j = 0; j < nt; ++j) {
-        ps.carry[s + j] = Ops::pack(carry);
-        mbar_arrive(&ps.cready[s + j]);
-        if (j + 1 < nt) carry = Ops::combine(carry, Ops::unpack(ps.agg[s + j]));
-      }
-    }
+    __syncwarp();  // every lane has read the unit's slots
+    if (lane == 0)
+      hand_on_carries<Ops>(
+          carry, nt, [&](int j) { return Ops::unpack(ps.agg[s + j]); },
+          [&](int j, Pub c) {
+            ps.carry[s + j] = Ops::pack(c);
+            mbar_arrive(&ps.cready[s + j]);
+          });
     __syncwarp();
   }
 }
