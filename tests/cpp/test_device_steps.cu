@@ -1,10 +1,16 @@
 // Steps of the device code that also compile for the host, run on the CPU:
 //   carries   the hand-over of a look-back unit's carries, with every slot
-//             taken again at the moment it is handed on.
+//             taken again at the moment it is handed on;
+//   windows   the splits and windows of a merge tile whose keys are in order,
+//             in no order, or have NaNs among them: every read inside the tile.
 // Prints one line per check and ALL PASSED when every check holds.
+#include "b2p_device/merge.cuh"
 #include "b2p_device/pipe.cuh"
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
+#include <random>
 #include <vector>
 
 namespace {
@@ -49,10 +55,88 @@ void carries() {
   check(ok, "carries of a unit when its slots are taken again at once");
 }
 
+// A position in an array of n keys (one more readable key after them when
+// `spare`): a read outside is counted, and gives the first key.
+struct Checked {
+  const float *base;
+  int at, n;
+  long long *outside;
+  Checked operator+(int k) const { return {base, at + k, n, outside}; }
+  Checked operator-(int k) const { return {base, at - k, n, outside}; }
+  Checked &operator+=(int k) { return at += k, *this; }
+  Checked &operator-=(int k) { return at -= k, *this; }
+  float operator[](int k) const {
+    const bool in = at + k >= 0 && at + k < n;
+    *outside += !in;
+    return base[in ? at + k : 0];
+  }
+};
+
+struct Before {
+  bool operator()(float x, float y) const { return x < y; }
+};
+
+// One staged tile of fp32 keys: every thread's split, and the window of every
+// thread that merge_window_inside lets use the network (i < ca: key i of a,
+// else key ITEMS - i of b, whose first one may be the key after b's last).
+void tile_windows(const std::vector<float> &a, const std::vector<float> &b, long long &outside, int &crossed) {
+  using Net = b2p::MergeNet<float>;
+  constexpr int ITEMS = Net::kItems, NT = Net::kThreads;
+  const int na = (int)a.size(), nb = (int)b.size(), cnt = na + nb;
+  std::vector<float> a1(a), b1(b);
+  a1.push_back(0.f);
+  b1.push_back(0.f);  // (the key after b's last)
+  const Checked sa{a1.data(), 0, na, &outside}, sb{b1.data(), 0, nb, &outside};
+  std::vector<int> lo(NT + 1, na);
+  for (int t = 0; t < NT; ++t) lo[t] = b2p::merge_tile_split<2048>(sa, sb, std::min(t * ITEMS, cnt), na, nb, Before{});
+  for (int t = 0; t < NT; ++t) {
+    const int d = std::min(t * ITEMS, cnt), ca = lo[t + 1] - lo[t];
+    if (d + ITEMS > cnt) continue;
+    if (!b2p::merge_window_inside<ITEMS>(ca, na - lo[t], nb - (d - lo[t]))) {
+      ++crossed;
+      continue;
+    }
+    const Checked wa = sa + lo[t], wb{b1.data(), d - lo[t] + ITEMS, nb + 1, &outside};
+    for (int i = 0; i <= ITEMS; ++i) (void)(i < ca ? wa + i : wb - i)[0];
+  }
+}
+
+void windows() {
+  std::mt19937 rng(1);
+  const int tile = b2p::MergeNet<float>::kTile;
+  for (int kind = 0; kind < 4; ++kind) {
+    long long outside = 0;
+    int crossed = 0;
+    for (int rep = 0; rep < 60; ++rep) {
+      const int cnt = rep % 3 ? tile : 1 + (int)(rng() % tile);
+      const int na = rep % 5 == 0 ? 0 : rep % 5 == 1 ? cnt : (int)(rng() % (cnt + 1));
+      std::vector<float> x(cnt);
+      for (float &v : x) v = (float)(int)(rng() % 20001) - 10000.f;
+      std::vector<float> a(x.begin(), x.begin() + na), b(x.begin() + na, x.end());
+      if (kind != 1) {
+        std::sort(a.begin(), a.end());
+        std::sort(b.begin(), b.end());
+      }
+      if (kind >= 2)  // NaNs at the end (2) or anywhere (3)
+        for (std::vector<float> *s : {&a, &b}) {
+          const size_t m = s->size(), from = kind == 2 ? m - m / 7 : 0;
+          for (size_t i = from; i < m; ++i)
+            if (kind == 2 || rng() % 9 == 0) (*s)[i] = NAN;
+        }
+      tile_windows(a, b, outside, crossed);
+    }
+    static const char *name[4] = {"windows, keys in order", "windows, keys in no order", "windows, NaNs at the end",
+                                  "windows, NaNs anywhere"};
+    printf("(%d threads merge serially) ", crossed);
+    check(outside == 0 && (kind == 0) == (crossed == 0), name[kind]);
+  }
+}
+
 }  // namespace
 
 int main() {
   carries();
+  windows();
   if (g_failed == 0) printf("ALL PASSED\n");
   return g_failed != 0;
 }

@@ -253,3 +253,28 @@ def test_merge_tile_edges(dev, code, desc):
                 out = torch.empty(total + off, dtype=dev_t(x[:1].copy()).dtype, device="cuda")[off:]
                 C.merge(dev_t(a), dev_t(b), out=out, descending=desc)
                 assert same_bits(out.cpu().numpy(), O.merge(a, b, desc)), (total, na, kind)
+
+
+@pytest.mark.parametrize("code", [C.F32, C.F64])
+@pytest.mark.parametrize("desc", [False, True])
+def test_merge_with_nans_writes_only_keys(dev, code, desc):
+    """NaNs compare as unordered, at the end of a side or anywhere in it, so
+    the order of the result is not specified; every key that it holds is one
+    of the inputs' keys.  Less than a tile, several tiles, and numbers of
+    tiles on both sides of the limit where a partition warp takes 32 of them."""
+    dt, bits = (torch.float32, torch.int32) if code == C.F32 else (torch.float64, torch.int64)
+    tile = 4960 if code == C.F32 else 2400
+    g = torch.Generator(device="cuda").manual_seed(600 + code + 10 * desc)
+    for total in (tile - 1, tile, 7 * tile + 5, 3000 * tile, 3000 * tile + 1):
+        for na in (total // 2, total // 9):
+            for where in ("end", "anywhere"):
+                sides = []
+                for n in (na, total - na):
+                    x = torch.sort(torch.randn(n, generator=g, device="cuda", dtype=dt), descending=desc)[0]
+                    if where == "end":
+                        x[n - n // 7:] = float("nan")
+                    else:
+                        x[torch.rand(n, generator=g, device="cuda") < 0.1] = float("nan")
+                    sides.append(x)
+                out = C.merge(*sides, descending=desc)
+                assert torch.isin(out.view(bits), torch.cat(sides).view(bits)).all(), (total, na, where)
