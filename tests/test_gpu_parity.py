@@ -592,3 +592,42 @@ def test_pipelined_scan_special_values(dev, code):
             assert torch.isfinite(got[:start]).all()
         inc = C.inclusive_scan(y)[:at].to(torch.float64)
         assert ((inc - ref[:at]).abs() <= 1e-6 * ref[:at]).all()
+
+
+@pytest.mark.parametrize("busy", ["elementwise", "sort", "scans"])
+def test_small_look_back_calls_beside_another_stream(dev, busy):
+    """Scans and copy_if whose blocks all fit on an empty GPU, while another
+    stream's work holds most of it (elementwise kernels, a sort's persistent
+    blocks, or look-back calls of its own), so that their blocks start late
+    and not together: exact results, and no wait has run out."""
+    ours, other = torch.cuda.Stream(), torch.cuda.Stream()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    big = torch.randint(0, 1 << 30, (1 << 26,), generator=g, device="cuda", dtype=torch.int32)
+    x = torch.randint(0, 1 << 20, ((1 << 20) + 3,), generator=g, device="cuda", dtype=torch.int32)
+    ref = torch.cumsum(x, 0).to(torch.int32)
+    keep = x[(x & 7) < 3]
+    torch.cuda.synchronize()
+    for n in (5000, 300007, (1 << 20) + 3):
+        kept = int(((x[:n] & 7) < 3).sum())
+        torch.cuda.synchronize()
+        if busy == "elementwise":
+            with torch.cuda.stream(other):
+                y = big.float()
+                for _ in range(6):
+                    y = torch.sin(y)
+        elif busy == "sort":
+            with torch.cuda.stream(other):
+                y = big.clone()
+            C.sort_(y, stream=other)
+        got = []
+        for _ in range(40):
+            with torch.cuda.stream(ours):
+                got.append((C.inclusive_scan(x[:n], stream=ours), C.copy_if(x[:n], 7, C.CMP_LT, 3, stream=ours)))
+            if busy == "scans":
+                with torch.cuda.stream(other):
+                    y = C.inclusive_scan(x, stream=other)
+        torch.cuda.synchronize()
+        for s, (out, cnt) in got:
+            assert torch.equal(s, ref[:n]), n
+            assert int(cnt.item()) == kept and torch.equal(out[:kept], keep[:kept]), n
+        assert C.device_error(ours) == C.OK and C.device_error(other) == C.OK
