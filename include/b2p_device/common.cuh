@@ -68,7 +68,8 @@ __device__ __forceinline__ void st_stream_v4(void *p, uint4 v) {
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// early = false: an ordinary launch of such a kernel.
+// early = false: an ordinary launch of such a kernel.  An error is returned,
+// not also left for the next cudaGetLastError of the process to find.
 template <class... P, class... A>
 inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
                                     cudaStream_t st, A... args) {
@@ -82,7 +83,9 @@ inline cudaError_t launch_dependent(bool early, void (*kernel)(P...), unsigned g
   c.stream = st;
   c.attrs = &attr;
   c.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // Tile status word of the single-pass look-back: {payload, meta} read and

@@ -11,6 +11,7 @@ duplicates-heavy keys, and at 2^28 keys size-independent properties
 (sorted, the same multiset as the input: the sum of the keys and the
 histogram of their top byte).
 """
+import ctypes
 import os
 
 import numpy as np
@@ -278,3 +279,32 @@ def test_merge_with_nans_writes_only_keys(dev, code, desc):
                     sides.append(x)
                 out = C.merge(*sides, descending=desc)
                 assert torch.isin(out.view(bits), torch.cat(sides).view(bits)).all(), (total, na, where)
+
+
+@pytest.mark.parametrize("op", ["merge", "sort"])
+def test_a_failed_launch_is_reported_once(dev, op):
+    """A merge or sort on a stream whose capture has become invalid returns
+    ERR_CUDA, and leaves no error behind for the next caller of the CUDA
+    runtime to find."""
+    cudart = ctypes.CDLL("libcudart.so.12")
+    x = torch.sort(torch.randn(100000, device="cuda"))[0]
+    out = torch.empty(200000, device="cuda")
+    n = x.numel()
+    nbytes = C.lib().b2p_scratch_bytes(C.PRIM_SORT, C.F32, 2 * n, 0, C.AUTO)
+    tmp = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    handle = ctypes.c_void_p(st.cuda_stream)
+    assert cudart.cudaStreamBeginCapture(handle, 2) == 0  # relaxed: other streams' calls go on
+    assert cudart.cudaStreamSynchronize(handle) != 0  # not allowed: the capture is invalid from here on
+    cudart.cudaGetLastError()
+    if op == "merge":
+        status = C.lib().b2p_merge(C.F32, x.data_ptr(), n, x.data_ptr(), n, out.data_ptr(), 0, tmp.data_ptr(), nbytes,
+                                   handle)
+    else:
+        status = C.lib().b2p_sort(C.F32, x.data_ptr(), n, 0, tmp.data_ptr(), nbytes, handle)
+    left = cudart.cudaGetLastError()
+    graph = ctypes.c_void_p()
+    assert cudart.cudaStreamEndCapture(handle, ctypes.byref(graph)) != 0 and not graph
+    cudart.cudaGetLastError()
+    assert status == C.ERR_CUDA and left == 0
