@@ -203,6 +203,21 @@ __device__ __forceinline__ PairView<T> pair_of(const T *a, long long na, const T
   return v;
 }
 
+// Keys of the first range among a tile's cnt outputs, from the tile's start
+// (i0 and j0 of nA and nB keys) and the first range's index i1 where the tile
+// ends.  i1 - i0 for ordered ranges; ranges that are not (NaNs among the keys)
+// can give tile starts that cross, and the result then keeps the tile inside
+// both ranges.
+__host__ __device__ __forceinline__ int merge_tile_count(long long i0, long long i1, long long nA, long long j0,
+                                                         long long nB, int cnt) {
+  const long long low = cnt - (nB - j0), high = nA - i0;
+  long long n = i1 - i0;
+  n = n > low ? n : low;
+  n = n > 0 ? n : 0;
+  n = n < high ? n : high;
+  return (int)(n < cnt ? n : cnt);
+}
+
 template <class T, class Comp, bool PAIRS>
 __global__ void __launch_bounds__(256) merge_partition_kernel(const T *a, long long na, const T *b, long long nb,
                                                               long long run, long long ntiles, long long *splits,
@@ -237,9 +252,9 @@ __global__ void __launch_bounds__(kMergeThreads) merge_kernel(const T *a, long l
   const long long l1 = tile_end - v.base;
   const long long i0 = splits[blockIdx.x];
   const long long i1 = l1 == v.nA + v.nB ? v.nA : splits[blockIdx.x + 1];
-  const long long j0 = (d0 - v.base) - i0, j1 = l1 - i1;
-  const int na_t = (int)(i1 - i0), nb_t = (int)(j1 - j0);
-  const int cnt = na_t + nb_t;
+  const long long j0 = (d0 - v.base) - i0;
+  const int cnt = (int)(tile_end - d0);
+  const int na_t = merge_tile_count(i0, i1, v.nA, j0, v.nB, cnt), nb_t = cnt - na_t;
   if (cnt == kMergeTile) {
     // a full tile: every thread's ITEMS loads in flight at once
     const T *pa = A + i0, *pb = B + (j0 - na_t);
@@ -513,9 +528,7 @@ __global__ void __launch_bounds__(MergeNet<T>::kThreads, MergeNet<T>::kBlocksPer
   auto stage = [&](T *slots, long long tile, long long i0, long long i1, int &na_t, int &cnt, int &a0, int &b0) {
     const long long d0 = tile * TILE;
     cnt = (int)min((long long)TILE, total - d0);
-    // (the bounds hold by themselves for sorted inputs; for others they keep
-    // every access inside the inputs and the tile)
-    na_t = (int)min(max(i1 - i0, max(0ll, cnt - (nb - (d0 - i0)))), min((long long)cnt, na - i0));
+    na_t = merge_tile_count(i0, i1, na, d0 - i0, nb, cnt);
     const T *pa = a + i0, *pb = b + (d0 - i0);
     a0 = (int)(reinterpret_cast<uintptr_t>(pa) & 15) / (int)sizeof(T);
     const int shift_b = (int)(reinterpret_cast<uintptr_t>(pb) & 15) / (int)sizeof(T);

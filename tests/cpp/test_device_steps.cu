@@ -2,7 +2,9 @@
 //   carries   the hand-over of a look-back unit's carries, with every slot
 //             taken again at the moment it is handed on;
 //   windows   the splits and windows of a merge tile whose keys are in order,
-//             in no order, or have NaNs among them: every read inside the tile.
+//             in no order, or have NaNs among them: every read inside the tile;
+//   counts    the keys that a merge tile takes of each range, for tile starts
+//             in order and crossing: never more than there are.
 // Prints one line per check and ALL PASSED when every check holds.
 #include "b2p_device/merge.cuh"
 #include "b2p_device/pipe.cuh"
@@ -132,11 +134,37 @@ void windows() {
   }
 }
 
+// Tile starts of random places: each within its range (as merge_path keeps
+// it), the next tile's in order or not.
+void counts() {
+  std::mt19937 rng(2);
+  bool inside = true, same = true;
+  int crossing = 0;
+  for (int rep = 0; rep < 200000; ++rep) {
+    const long long nA = rng() % 5000, nB = rng() % 5000;
+    if (nA + nB == 0) continue;
+    const long long d0 = rng() % (nA + nB);
+    const int cnt = (int)std::min<long long>(1 + rng() % 4096, nA + nB - d0);
+    auto start = [&](long long d) {
+      const long long lo = std::max(0ll, d - nB), hi = std::min(d, nA);
+      return lo + (long long)(rng() % (hi - lo + 1));
+    };
+    const long long i0 = start(d0), i1 = start(d0 + cnt), j0 = d0 - i0, j1 = d0 + cnt - i1;
+    const int na = b2p::merge_tile_count(i0, i1, nA, j0, nB, cnt);
+    inside = inside && na >= 0 && na <= cnt && i0 + na <= nA && j0 + (cnt - na) <= nB;
+    if (i1 >= i0 && j1 >= j0) same = same && na == i1 - i0;
+    else ++crossing;
+  }
+  printf("(%d starts cross) ", crossing);
+  check(inside && same && crossing > 0, "keys of a merge tile");
+}
+
 }  // namespace
 
 int main() {
   carries();
   windows();
+  counts();
   if (g_failed == 0) printf("ALL PASSED\n");
   return g_failed != 0;
 }

@@ -308,3 +308,19 @@ def test_a_failed_launch_is_reported_once(dev, op):
     assert cudart.cudaStreamEndCapture(handle, ctypes.byref(graph)) != 0 and not graph
     cudart.cudaGetLastError()
     assert status == C.ERR_CUDA and left == 0
+
+
+@pytest.mark.parametrize("code", [C.F32, C.F64])
+@pytest.mark.parametrize("n", [5000, 20000, 32767])
+def test_sort_with_nans_writes_only_keys(dev, code, n):
+    """Sorts of several tiles below the radix sort's size, with NaNs anywhere:
+    the merge passes' runs are then in no order, and the order of the result
+    is not specified; every key that it holds is one of the input's."""
+    dt, bits = (torch.float32, torch.int32) if code == C.F32 else (torch.float64, torch.int64)
+    g = torch.Generator(device="cuda").manual_seed(700 + code)
+    for share in (0.001, 0.1, 0.9):
+        for desc in (False, True):
+            x = torch.randn(n, generator=g, device="cuda", dtype=dt)
+            x[torch.rand(n, generator=g, device="cuda") < share] = float("nan")
+            y = C.sort_(x.clone(), descending=desc)
+            assert torch.isin(y.view(bits), x.view(bits)).all(), (share, desc)
