@@ -160,7 +160,19 @@ __global__ void __launch_bounds__(kRadixThreads) radix_upsweep_kernel(const T *k
       }
     }
   }
-  for (i += t; i < b1; i += kRadixThreads) count(__ldcg(keys + i));
+  // what is left, or keys that are not 16-byte aligned: 4-byte keys with eight
+  // loads in flight (a last tile's counts: 300,000 int32 56 -> 47 us a sort;
+  // 3.6 M unaligned int64 got slower that way, 242 -> 254 us)
+  constexpr unsigned kLate = sizeof(T) == 4 ? 8 : 1;
+  for (i += t; i < b1; i += kLate * kRadixThreads) {
+    T k[kLate];
+#pragma unroll
+    for (unsigned r = 0; r < kLate; ++r)
+      if (i + r * kRadixThreads < b1) k[r] = __ldcg(keys + i + r * kRadixThreads);
+#pragma unroll
+    for (unsigned r = 0; r < kLate; ++r)
+      if (i + r * kRadixThreads < b1) count(k[r]);
+  }
   __syncthreads();
   for (unsigned d = t; d < kRadixBins; d += kRadixThreads) {
     unsigned c = 0;
@@ -238,19 +250,31 @@ __device__ __forceinline__ unsigned radix_stage(unsigned r, unsigned c) {
 // Bring tile `t0 .. t0 + count` of `in` into `buf`, block kb in row
 // (kb & 3) * 32 + kb / 4; keys past the end are `pad` (digit 255 in every
 // pass, so that they stay behind the tile's real keys).  Full tiles of
-// 16-byte aligned input come by cp.async.
-template <class T>
+// 16-byte aligned input come by cp.async, other tiles key by key.  ALONE: the
+// block has nothing to do until the tile is there, so a partial aligned tile
+// comes by cp.async too, up to the vector in which the input ends.  (Key by
+// key, one after the other, the last tile kept every pass waiting: 400,000
+// int32, 49 tiles, 72 us a sort and 49 with it.)
+template <class T, bool ALONE>
 __device__ __forceinline__ void radix_load_tile(char *buf, const T *in, unsigned t0, unsigned count, bool vec, T pad) {
-  constexpr unsigned K = kRadixItemBytes / sizeof(T), TILE = K * kDownThreads;
+  constexpr unsigned K = kRadixItemBytes / sizeof(T), TILE = K * kDownThreads, IPV = 16 / sizeof(T);
   const unsigned t = threadIdx.x;
-  if (vec && count == TILE) {
+  if (vec && (ALONE || count == TILE)) {
     const char *g = reinterpret_cast<const char *>(in + t0) + t * 16;
-    const unsigned c = t & 15u, row0 = ((t >> 4) & 3u) * 32u + (t >> 6);
+    const unsigned c = t & 15u, row0 = ((t >> 4) & 3u) * 32u + (t >> 6), nvec = count / IPV;
 #pragma unroll
     for (unsigned q = 0; q < 16; ++q) {
-      const unsigned d = (unsigned)__cvta_generic_to_shared(buf + radix_stage(row0 + 2 * q, c));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g + (size_t)q * kDownThreads * 16)
-                   : "memory");
+      char *const to = buf + radix_stage(row0 + 2 * q, c);
+      const unsigned v = q * kDownThreads + t;
+      if (!ALONE || v < nvec) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(to);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g + (size_t)q * kDownThreads * 16)
+                     : "memory");
+      } else {
+#pragma unroll
+        for (unsigned e = 0; e < IPV; ++e)
+          reinterpret_cast<T *>(to)[e] = v * IPV + e < count ? __ldcg(in + t0 + v * IPV + e) : pad;
+      }
     }
   } else {
     for (unsigned e = t; e < TILE; e += kDownThreads) {
@@ -326,7 +350,7 @@ __global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
   grid_wait();
   grid_trigger();
   if (tile_begin < tile_end)
-    radix_load_tile<T>(x, in, tile_begin * TILE, min(TILE, n - tile_begin * TILE), vec, pad);
+    radix_load_tile<T, true>(x, in, tile_begin * TILE, min(TILE, n - tile_begin * TILE), vec, pad);
 
   // next output slot of this thread's digits 2t and 2t + 1 in this chunk
   uint2 mine;
@@ -435,7 +459,7 @@ __global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
     __syncthreads();  // counters and prefixes are used up
 
     if (tile + 1 < tile_end)
-      radix_load_tile<T>(y, in, (tile + 1) * TILE, min(TILE, n - (tile + 1) * TILE), vec, pad);
+      radix_load_tile<T, false>(y, in, (tile + 1) * TILE, min(TILE, n - (tile + 1) * TILE), vec, pad);
 #pragma unroll
     for (unsigned j = 0; j < K; ++j) {
       const unsigned z = j % 2 ? pos[j / 2] >> 16 : pos[j / 2] & 0xffffu;
@@ -456,6 +480,7 @@ __global__ void __launch_bounds__(kDownThreads, kDownBlocksPerSm)
 #pragma unroll 16
       for (unsigned r = 0; r < K; ++r) put(r);
     } else {
+#pragma unroll 4
       for (unsigned r = 0; r * kDownThreads + t < count; ++r) put(r);
     }
     __syncthreads();
@@ -506,17 +531,20 @@ int launch_radix_sort(T *keys, size_t n, bool desc, void *scratch, size_t scratc
   if (cudaFuncSetAttribute((const void *)radix_downsweep_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return B2P_ERR_CUDA;
-  // One tile per block: 3 P launches of 3 to 10 us each, which overlap their
-  // start with the end of the one before (1,000,003 doubles: 156 -> 144 us).
-  // Longer launches start in order: early blocks of the next kernel keep an SM
-  // from taking its share (2^28 int32: 3.81 ms against 4.18).
-  const bool early = l.chunk == 1;
+  // One tile per block: 3 P launches of 3 to 10 us each, whose spine starts
+  // while the upsweep ends (1,000,003 doubles 116 -> 113 us, 400,000 103 -> 97).
+  // Up to 32 tiles the other two do so as well (131,072 int32 46 -> 43 us).  With
+  // more, blocks that wait take places on few SMs, where they then work several
+  // to an SM while others have none: 196,608 int64 87 us against 110 with all
+  // early, 1,000,003 int32 52 against 66.  Launches of several tiles per block
+  // start in order (2^28 int32: 3.81 ms against 4.18).
+  const bool spine_early = l.chunk == 1, early = spine_early && l.blocks <= 32;
   const T *src = keys;
   T *dst = buf;
   for (int p = 0; p < P; ++p) {
     if (launch_dependent(early, radix_upsweep_kernel<T>, l.blocks, kRadixThreads, 0, st, src, (unsigned)n, desc, p, l.chunk,
                          counts) != cudaSuccess ||
-        launch_dependent(early, radix_spine_kernel, kRadixBins, kRadixSpineThreads, 0, st, counts, l.blocks, totals) !=
+        launch_dependent(spine_early, radix_spine_kernel, kRadixBins, kRadixSpineThreads, 0, st, counts, l.blocks, totals) !=
             cudaSuccess ||
         launch_dependent(early, radix_downsweep_kernel<T>, l.blocks, kDownThreads, smem, st, src, dst, (unsigned)n, desc, p,
                          l.chunk, counts, totals, radix_pad<T>(desc)) != cudaSuccess)
