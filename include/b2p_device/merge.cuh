@@ -643,9 +643,26 @@ int launch_merge(const T *a, size_t na, const T *b, size_t nb, T *out, const Com
   return cudaGetLastError() == cudaSuccess ? B2P_OK : B2P_ERR_CUDA;
 }
 
-// The same for standard keys, ascending or descending.
-constexpr long long kMergeWarpTiles = 3000;
+// Whether a merge of standard keys takes the kernels below or launch_merge().
+// The network's tiles are larger, so the GPU fills later: up to 2^18 keys that
+// does not matter (one tile per SM or fewer) and the two kernels overlap their
+// starts, from 7 x 2^18 on the cheaper merge outweighs it, between them
+// launch_merge() is the faster one (600,000 + 500,000 int32 7.7 us against 9.1,
+// int64 9.6 against 9.9; 1,000,000 + 900,000 int32 10.5 against 9.2).  8-byte
+// keys that come nearly all from one side are a copy, bound by L2 while it
+// holds them: 3,000,000 + 3,000 int64 13.7 against 15.2, 14,500,000 + 3,900 54.7
+// against 56.1, 25,000,000 + 3,000 94.8 against 93.9.
+constexpr long long kMergeEarlyKeys = 1ll << 18, kMergeNetKeys = 7ll << 18, kMergeLopsidedKeys = 1ll << 24;
 
+template <class T>
+inline bool merge_by_network(size_t na, size_t nb) {
+  const long long total = (long long)(na + nb), small = (long long)std::min(na, nb);
+  if (total <= kMergeEarlyKeys) return true;
+  if (sizeof(T) == 8 && small < total / 64 && total < kMergeLopsidedKeys) return false;
+  return total >= kMergeNetKeys;
+}
+
+// The same for standard keys, ascending or descending.
 template <class T, bool DESC>
 int launch_merge_keys(const T *a, size_t na, const T *b, size_t nb, T *out, void *scratch, size_t scratch_bytes,
                       int sm_count, cudaStream_t st) {
@@ -655,17 +672,23 @@ int launch_merge_keys(const T *a, size_t na, const T *b, size_t nb, T *out, void
   if (tiles > 0x7fffffffLL / 32) return B2P_ERR_INVALID_ARG;
   if (!scratch || scratch_bytes < merge_scratch_bytes<T>((size_t)total) - 256) return B2P_ERR_SCRATCH;
   long long *splits = reinterpret_cast<long long *>(scratch);
-  // a search per warp while the tiles are few (latency), 32 tiles a warp beyond
-  // (2083 tiles of int64: 28 us against 35; 3427 of fp32: 64 against 56)
-  // (a merge of many tiles starts in order, 260 us against 290 for 133 M floats:
-  // early blocks keep an SM from taking its share)
-  const bool few = tiles <= kMergeWarpTiles;
-  const auto partition = few ? merge_keys_partition_kernel<T, DESC, 1> : merge_keys_partition_kernel<T, DESC, 32>;
+  // Tiles per partition warp: one search per warp while the tiles are few
+  // (latency), more as their scattered reads add up.  10.5 M + 10.5 M int32 (4,234
+  // tiles) 58.0 us with 1, 57.6 with 8, 64.0 with 32; 25 M + 25 M (10,081 tiles)
+  // 133, 109, 114; 133 M (26,882 tiles) 308, 259, 255.
+  const int per_warp = tiles <= 4096 ? 1 : tiles <= 16384 ? 8 : 32;
+  const auto partition = per_warp == 1   ? merge_keys_partition_kernel<T, DESC, 1>
+                         : per_warp == 8 ? merge_keys_partition_kernel<T, DESC, 8>
+                                         : merge_keys_partition_kernel<T, DESC, 32>;
   const long long grid = std::min<long long>(tiles, (long long)sm_count * MergeNet<T>::kBlocksPerSm);
-  if (launch_dependent(few, partition, (unsigned)(few ? (tiles + 3) / 4 : (tiles + 127) / 128), 128, 0, st, a,
+  // Started while the kernel before ends only when the SMs have room for both:
+  // an early partition of the next merge keeps merge blocks of this one waiting
+  // (2,000,000 + 1,500,000 int32 12.0 us in order, 19.1 early).
+  const bool early = total <= kMergeEarlyKeys;
+  if (launch_dependent(early, partition, (unsigned)((tiles + 4 * per_warp - 1) / (4 * per_warp)), 128, 0, st, a,
                        (long long)na, b, (long long)nb, tiles, splits) != cudaSuccess ||
-      launch_dependent(few, merge_keys_kernel<T, DESC>, (unsigned)grid, MergeNet<T>::kThreads, 0, st, a, (long long)na, b,
-                       (long long)nb, out, tiles, (const long long *)splits) != cudaSuccess)
+      launch_dependent(early, merge_keys_kernel<T, DESC>, (unsigned)grid, MergeNet<T>::kThreads, 0, st, a, (long long)na,
+                       b, (long long)nb, out, tiles, (const long long *)splits) != cudaSuccess)
     return B2P_ERR_CUDA;
   return B2P_OK;
 }

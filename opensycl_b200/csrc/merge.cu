@@ -24,6 +24,9 @@ int merge_t(const void *a, size_t na, const void *b, size_t nb, void *out, bool 
             cudaStream_t st) {
   const T *pa = reinterpret_cast<const T *>(a), *pb = reinterpret_cast<const T *>(b);
   T *po = reinterpret_cast<T *>(out);
+  if (!merge_by_network<T>(na, nb))
+    return desc ? launch_merge(pa, na, pb, nb, po, Greater<T>{}, scratch, sb, st)
+                : launch_merge(pa, na, pb, nb, po, Less<T>{}, scratch, sb, st);
   const int sms = device_info().sm_count;
   return desc ? launch_merge_keys<T, true>(pa, na, pb, nb, po, scratch, sb, sms, st)
               : launch_merge_keys<T, false>(pa, na, pb, nb, po, scratch, sb, sms, st);

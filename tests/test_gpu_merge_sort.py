@@ -324,3 +324,21 @@ def test_sort_with_nans_writes_only_keys(dev, code, n):
             x[torch.rand(n, generator=g, device="cuda") < share] = float("nan")
             y = C.sort_(x.clone(), descending=desc)
             assert torch.isin(y.view(bits), x.view(bits)).all(), (share, desc)
+
+
+@pytest.mark.parametrize("code", [C.I32, C.F64])
+def test_merge_at_the_route_rules(dev, code):
+    """Totals on both sides of every rule of the merge's route (2^18 and 7 x 2^18
+    keys, the lopsided 8-byte merges up to 2^24 keys, 4,096 and 16,384 tiles),
+    sides of equal and of very different length, both orders: the bits of the
+    sorted whole."""
+    dt = torch.int32 if code == C.I32 else torch.float64
+    tile = 4960 if code == C.I32 else 2400
+    g = torch.Generator(device="cuda").manual_seed(code)
+    for total in (1 << 18, 7 << 18, 1 << 24, 4096 * tile, 16384 * tile):
+        for n in (total - 1, total, total + 1):
+            x = torch.randint(-(1 << 31), 1 << 31, (n,), generator=g, device="cuda").to(dt)
+            for na, desc in ((n // 2, False), (n // 65, True), (n - 3, False)):
+                a, b = torch.sort(x[:na], descending=desc)[0], torch.sort(x[na:], descending=desc)[0]
+                ref = torch.sort(x, descending=desc)[0]
+                assert torch.equal(C.merge(a, b, descending=desc), ref), (n, na, desc)
