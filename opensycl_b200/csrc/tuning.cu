@@ -54,22 +54,30 @@ int heuristic_config(int prim, int dtype, size_t n, int64_t nseg) {
   case B2P_PRIM_COPY_IF: {
     // The pipelined (TMA) kernel once its blocks have several tiles each: a scan
     // beyond 16 MiB (2^22 int32: 13.8 us against 13.0 us of the look-back
-    // kernel; 5 x 2^20: 15.0 against 17.4), copy_if beyond 13 MiB of uint32
-    // (3 x 2^20: 15.2 against 13.3; 2^22: 15.8 against 20.3) and 16 MiB of int64
-    // (2^21: 15.8 against 15.4; 3 x 2^20: 17.5 against 21.3).
+    // kernel; 5 x 2^20: 15.0 against 17.4), copy_if beyond 13.75 MiB, where the
+    // look-back kernel's 64 KiB blocks, three to an SM, no longer all run at once
+    // (uint32, 3.5 M: 15.9 against 14.3, 2^22: 15.7 against 20.3; int64, 1.8 M:
+    // 15.5 against 13.2, 2.1 M: 15.5 against 16.0).
     const bool scan = prim == B2P_PRIM_SCAN;
-    if (scan ? n * acc_size(dtype) > (16u << 20) : bytes > ((es == 8 ? 16u : 13u) << 20))
-      return cfg(1, 256, es == 8 ? 16 : 32);
+    if (scan ? n * acc_size(dtype) > (16u << 20) : bytes > (55u << 18)) return cfg(1, 256, es == 8 ? 16 : 32);
     // Below, one look-back tile per block: the smallest tile that still leaves
     // at most about one tile per SM, because the time is the latency of one
-    // tile and the look-back over the others (2^16 int32: 5.5 us with 2048
+    // tile and the look-back over the others (2^16 int32: 5.9 us with 2048
     // elements, 10.5 us with 8192; 2^19: 7.2 us with 4096, 11.3 us with 8192;
     // 2^21: 10.0 us with 512 x 16, 12.4 us with 256 x 32).
     if (n <= (1u << 18)) return es == 2 ? cfg(0, 256, 8) : cfg(0, 512, 4);
     if (n <= (1u << 19)) return es == 4 ? cfg(0, 1024, 4) : cfg(0, 512, 8);
-    if (scan && es == 8) return cfg(0, 256, 16);
-    if (n <= (1u << 20) || es == 8) return cfg(0, 1024, 8);
-    return n <= (1u << 21) ? cfg(0, 512, 16) : cfg(0, 256, 32);
+    // 8-byte scans, copy_if of 8-byte elements: one 1024 x 8 block per SM up to
+    // 148 of them (int64, 1.5 M: 15.0 us with that, 12.8 with 256 x 16).  FP64
+    // scans beyond 2^20: 1.5 M 13.9 us with 256 x 32, 16.8 with 256 x 16.
+    if (es == 8 && scan) return dtype == B2P_F64 && n > (1u << 20) ? cfg(0, 256, 32) : cfg(0, 256, 16);
+    if (es == 8) return n <= (37u << 15) ? cfg(0, 1024, 8) : cfg(0, 256, 16);
+    if (n <= (1u << 20)) return cfg(0, 1024, 8);
+    // 512 x 16 while two blocks per SM hold the tiles (copy_if, 2^21: 10.3 us
+    // against 13.0 with 256 x 32; 2.5 M: 14.6 against 13.1), for the floats' scans
+    // not as long (bf16, 1.5 M: 10.5 against 10.9, 2^21: 12.3 against 11.6).
+    const bool compensated = scan && dtype_is_float(dtype);
+    return n <= (compensated ? 7u << 18 : scan ? 1u << 21 : 37u << 16) ? cfg(0, 512, 16) : cfg(0, 256, 32);
   }
   case B2P_PRIM_HISTOGRAM:
     return cfg(1, 1024, 32);

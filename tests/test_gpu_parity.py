@@ -631,3 +631,29 @@ def test_small_look_back_calls_beside_another_stream(dev, busy):
             assert torch.equal(s, ref[:n]), n
             assert int(cnt.item()) == kept and torch.equal(out[:kept], keep[:kept]), n
         assert C.device_error(ours) == C.OK and C.device_error(other) == C.OK
+
+
+@pytest.mark.parametrize("code", [C.U32, C.I64, C.F32, C.BF16, C.F64])
+def test_scan_and_copy_if_at_the_wave_rules(dev, code):
+    """Sizes on both sides of the rules that count the look-back blocks an SM
+    holds (7 x 2^18, 37 x 2^15, 37 x 2^16, 110 x 2^14 and 55 x 2^16 elements): scans
+    against torch's cumulative sum, copy_if against a mask, integers exact,
+    floats within 1e-6."""
+    g = torch.Generator(device="cuda").manual_seed(code)
+    for edge in (1 << 20, 37 << 15, 110 << 14, 7 << 18, 1 << 21, 37 << 16, 55 << 16):
+        for n in (edge, edge + 1):
+            if code in (C.U32, C.I64):
+                x = torch.randint(0, 1 << 20, (n,), generator=g, device="cuda")
+                ref = torch.cumsum(x, 0)
+                y = x if code == C.I64 else x.to(torch.uint32)
+                got = C.inclusive_scan(y).to(torch.int64)
+                assert torch.equal(got, ref if code == C.I64 else ref & 0xFFFFFFFF), n
+                out, cnt = C.copy_if(y, 7, C.CMP_LT, 5)
+                keep, k = x[(x & 7) < 5], int(cnt.item())
+                assert k == keep.numel() and torch.equal(out[:k].to(torch.int64), keep), n
+            else:
+                dt = {C.F32: torch.float32, C.BF16: torch.bfloat16, C.F64: torch.float64}[code]
+                x = torch.rand(n, generator=g, device="cuda").to(dt)
+                ref = torch.cumsum(x.to(torch.float64), 0)
+                got = C.inclusive_scan(x).to(torch.float64)
+                assert ((got - ref).abs() <= 1e-6 * ref.abs() + 1e-30).all(), n
