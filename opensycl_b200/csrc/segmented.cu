@@ -549,6 +549,7 @@ struct b2p_plan_s {
   int64_t nseg = 0;
   double bytes = 0;   // algorithmic bytes of one launch
   void *scratch = nullptr;
+  int64_t *offsets = nullptr;  // the plan's copy of offsets in pageable host memory
   size_t scratch_bytes = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -597,6 +598,16 @@ int b2p_plan_segmented(b2p_plan *plan, int prim, int dtype, int op, const void *
   pl->scratch_bytes = kScratchPrefix + np * (sizeof(StatusWord) + sizeof(Piece));
   if (flat) pl->scratch_bytes = std::max(pl->scratch_bytes, segmented_tma_scratch(total_elems, lc.block, lc.items));
   e = cudaMalloc(&pl->scratch, pl->scratch_bytes);
+  cudaPointerAttributes where;
+  if (e == cudaSuccess) e = cudaPointerGetAttributes(&where, offsets);
+  if (e == cudaSuccess && where.type == cudaMemoryTypeUnregistered) {
+    // offsets in pageable host memory: the records kernel and the plan's
+    // launches read the plan's copy
+    e = cudaMalloc(&pl->offsets, h.size() * sizeof(int64_t));
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(pl->offsets, h.data(), h.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st);
+    offsets = pl->offsets;
+  }
   if (e != cudaSuccess) {
     b2p_plan_destroy(pl);
     return cuda_status(e);
@@ -705,6 +716,7 @@ void b2p_plan_destroy(b2p_plan plan) {
   if (plan->exec) cudaGraphExecDestroy(plan->exec);
   if (plan->graph) cudaGraphDestroy(plan->graph);
   if (plan->scratch) cudaFree(plan->scratch);
+  if (plan->offsets) cudaFree(plan->offsets);
   delete plan;
 }
 

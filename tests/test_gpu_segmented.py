@@ -209,3 +209,31 @@ def test_segmented_reduce_sixteen_stage_tiles(dev):
     ref = total[offsets[1:]] - total[offsets[:-1]]
     got = C.segmented_reduce(x, offsets, config=cfg).double()
     assert ((got - ref).abs() <= 1e-6 * ref + 1e-6).all()
+
+
+@pytest.mark.parametrize("prim", [C.PRIM_SEG_REDUCE, C.PRIM_SEG_SCAN])
+@pytest.mark.parametrize("shape", ["long", "many", "min"])
+def test_plan_with_offsets_in_host_memory(dev, prim, shape):
+    """A plan takes offsets in pageable host memory: long segments (boundary
+    records), hundreds of boundaries in a tile (offsets read by the launch),
+    and an operator of the piece kernel.  The offsets may change afterwards."""
+    rng = np.random.default_rng(11)
+    lens = rng.integers(20000, 40000, 40) if shape != "many" else rng.integers(0, 30, 20000)
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    op = C.MIN if shape == "min" else C.SUM
+    x = values(rng, C.I64, int(offs[-1]))
+    ref = O.segmented_reduce(C.I64, op, x, offs) if prim == C.PRIM_SEG_REDUCE else \
+        O.segmented_scan(C.I64, op, True, x, offs)
+    xd = torch.from_numpy(x).cuda()
+    out = torch.zeros(ref.size, dtype=torch.int64, device="cuda")
+    plan, st = ctypes.c_void_p(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    host = offs.copy()
+    C.check(C.lib().b2p_plan_segmented(ctypes.byref(plan), prim, C.I64, op, xd.data_ptr(), out.data_ptr(),
+                                       host.ctypes.data, lens.size, x.size, C.AUTO, st))
+    host[:] = -1
+    for _ in range(2):
+        out.zero_()
+        C.check(C.lib().b2p_plan_launch(plan, st))
+        assert np.array_equal(out.cpu().numpy(), ref)
+    torch.cuda.synchronize()
+    C.lib().b2p_plan_destroy(plan)
