@@ -261,10 +261,17 @@ def _aligned_ptr(buf) -> int:
     return (p + 255) & ~255
 
 
-def scratch_for(prim: int, code: int, n: int, nseg: int = 0, config: int = AUTO, stream=None):
+def _scratch(prim: int, code: int, n: int, nseg: int, config: int, stream):
+    """(address, bytes) of the stream's scratch for a call."""
     nbytes = lib().b2p_scratch_bytes(prim, code, n, nseg, config)
     buf = Scratch.get(nbytes + 256, stream)
     return (buf.data_ptr() + 255) & ~255, buf.numel() - 256
+
+
+def scratch_for(prim: int, code: int, n: int, nseg: int = 0, config: int = AUTO, stream=None):
+    """The stream's scratch for a call: its pointer (c_void_p) and bytes."""
+    sp, sb = _scratch(prim, code, n, nseg, config, stream)
+    return ctypes.c_void_p(sp), sb
 
 
 def _result(n: int, init, code: int, x):
@@ -300,7 +307,7 @@ def reduce(x, op="sum", init=0, out=None, config: int = AUTO, stream=None):
     if out is None:
         out = _result(n, init, code, x)
     _, ip = _init_ptr(code, init)
-    sp, sb = scratch_for(PRIM_REDUCE, code, n, 0, config, stream)
+    sp, sb = _scratch(PRIM_REDUCE, code, n, 0, config, stream)
     _call(lib().b2p_reduce, "b2p_reduce", code, opc, x.data_ptr(), n, out.data_ptr(), ip, sp, sb, config,
           _stream_of(stream)[1])
     return out
@@ -311,7 +318,7 @@ def dot(a, b, init=0.0, out=None, config: int = AUTO, stream=None):
     if out is None:
         out = _result(n, init, code, a)
     _, ip = _init_ptr(code, init)
-    sp, sb = scratch_for(PRIM_DOT, code, n, 0, config, stream)
+    sp, sb = _scratch(PRIM_DOT, code, n, 0, config, stream)
     _call(lib().b2p_dot, "b2p_dot", code, a.data_ptr(), b.data_ptr(), n, out.data_ptr(), ip, sp, sb, config,
           _stream_of(stream)[1])
     return out
@@ -323,7 +330,7 @@ def scan(x, inclusive=True, op="sum", init=None, out=None, config: int = AUTO, s
     if out is None:
         out = _t().torch.empty(n, dtype=_t().acc[code], device=x.device)
     _, ip = _init_ptr(code, init)
-    sp, sb = scratch_for(PRIM_SCAN, code, n, 0, config, stream)
+    sp, sb = _scratch(PRIM_SCAN, code, n, 0, config, stream)
     _call(lib().b2p_scan, "b2p_scan", code, opc, int(bool(inclusive)), x.data_ptr(), out.data_ptr(), n, ip, sp, sb,
           config, _stream_of(stream)[1])
     return out
@@ -345,7 +352,7 @@ def copy_if(x, mask, cmp, rhs, out=None, count=None, config: int = AUTO, stream=
         out = _torch().empty_like(x)
     if count is None:
         count = zeros(1, _torch().uint64, x.device)
-    sp, sb = scratch_for(PRIM_COPY_IF, code, n, 0, config, stream)
+    sp, sb = _scratch(PRIM_COPY_IF, code, n, 0, config, stream)
     _call(lib().b2p_copy_if, "b2p_copy_if", code, x.data_ptr(), out.data_ptr(), n, mask, cmp, rhs, count.data_ptr(),
           sp, sb, config, _stream_of(stream)[1])
     return out, count
@@ -396,7 +403,7 @@ def segmented_reduce(x, offsets, op="sum", init=None, out=None, config: int = AU
     if out is None:
         out = _torch().empty(nseg, dtype=acc_torch_dtype(code), device=x.device)
     _, ip = _init_ptr(code, init)
-    sp, sb = scratch_for(PRIM_SEG_REDUCE, code, n, nseg, config, stream)
+    sp, sb = _scratch(PRIM_SEG_REDUCE, code, n, nseg, config, stream)
     _call(lib().b2p_segmented_reduce, "b2p_segmented_reduce", code, opc, x.data_ptr(), offsets.data_ptr(), nseg,
           out.data_ptr(), ip, sp, sb, config, _stream_of(stream)[1])
     return out
@@ -410,7 +417,7 @@ def segmented_scan(x, offsets, inclusive=True, op="sum", init=None, out=None, co
     if out is None:
         out = _torch().empty(n, dtype=acc_torch_dtype(code), device=x.device)
     _, ip = _init_ptr(code, init)
-    sp, sb = scratch_for(PRIM_SEG_SCAN, code, n, nseg, config, stream)
+    sp, sb = _scratch(PRIM_SEG_SCAN, code, n, nseg, config, stream)
     _call(lib().b2p_segmented_scan, "b2p_segmented_scan", code, opc, int(bool(inclusive)), x.data_ptr(),
           out.data_ptr(), offsets.data_ptr(), nseg, ip, sp, sb, config, _stream_of(stream)[1])
     return out

@@ -121,3 +121,14 @@ def test_calls_without_device_fail_cleanly():
     rc = L.b2p_reduce(C.F32, C.SUM, p, 64, out.ctypes.data_as(ctypes.c_void_p), None, p, 256, 0, None)
     assert rc != C.OK
     assert out[0] == 0
+
+
+def test_scratch_for_returns_a_pointer_and_bytes(monkeypatch):
+    """The scratch helper that programs use beside the C-ABI: a c_void_p, 256-byte
+    aligned inside the stream's buffer, and the bytes behind it."""
+    import torch
+    buf = torch.zeros(1 << 20, dtype=torch.uint8)
+    monkeypatch.setattr(C.Scratch, "get", classmethod(lambda cls, nbytes, stream=None: buf))
+    sp, sb = C.scratch_for(C.PRIM_REDUCE, C.F32, 1024)
+    assert isinstance(sp, ctypes.c_void_p) and sp.value % 256 == 0
+    assert buf.data_ptr() <= sp.value and sp.value + sb <= buf.data_ptr() + buf.numel()
