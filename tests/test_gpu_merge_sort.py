@@ -342,3 +342,44 @@ def test_merge_at_the_route_rules(dev, code):
                 a, b = torch.sort(x[:na], descending=desc)[0], torch.sort(x[na:], descending=desc)[0]
                 ref = torch.sort(x, descending=desc)[0]
                 assert torch.equal(C.merge(a, b, descending=desc), ref), (n, na, desc)
+
+
+@pytest.mark.parametrize("n", [100003, 1000003])
+def test_sort_and_merge_in_a_captured_graph(dev, n):
+    """Sorts and merges whose kernels start early, captured into a graph: right
+    behind a copy, behind another call's last kernel, as the first work of a
+    forked stream and as the first after two streams join.  Replays on new
+    inputs sort and merge those."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+
+    def new(k):
+        return torch.randint(-(1 << 31), 1 << 31, (k,), generator=g, device="cuda", dtype=torch.int32)
+
+    x, a, b = new(n), torch.sort(new(n))[0], torch.sort(new(n // 2))[0]
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    ab, aab = torch.empty(n + n // 2, dtype=torch.int32, device="cuda"), torch.empty(2 * n + n // 2, dtype=torch.int32,
+                                                                                    device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            C.merge(a, b, out=ab, stream=side)
+            C.merge(a, ab, out=aab, stream=side)
+        y.copy_(x)
+        C.sort_(y, stream=main)
+        z.copy_(y)
+        main.wait_stream(side)
+        C.sort_(z, descending=True, stream=main)
+    for _ in range(3):
+        x.copy_(new(n))
+        a.copy_(torch.sort(new(n))[0])
+        b.copy_(torch.sort(new(n // 2))[0])
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, torch.sort(x)[0]) and torch.equal(z, torch.sort(x, descending=True)[0])
+        assert torch.equal(ab, torch.sort(torch.cat([a, b]))[0])
+        assert torch.equal(aab, torch.sort(torch.cat([a, a, b]))[0])

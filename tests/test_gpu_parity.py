@@ -657,3 +657,105 @@ def test_scan_and_copy_if_at_the_wave_rules(dev, code):
                 ref = torch.cumsum(x.to(torch.float64), 0)
                 got = C.inclusive_scan(x).to(torch.float64)
                 assert ((got - ref).abs() <= 1e-6 * ref.abs() + 1e-30).all(), n
+
+
+def canonical_sum(x, init, chains, lift, off_bytes):
+    """The canonical sum of a 1-D array as numpy restates it: runs of 32 lanes x
+    16 vectors of 16 bytes, `chains` accumulators per lane, a lane butterfly, the
+    512-wide halving tree over the runs, then head, body and tail.  fp32 and
+    bf16 (chains 2 and 4) accumulate in double-float, fp64 plainly."""
+    df = chains > 1
+    ft = np.float32 if df else np.float64
+
+    def two_sum(a, b):
+        s = a + b
+        bp = s - a
+        return s, (a - (s - bp)) + (b - bp)
+
+    def add(acc, v):
+        if not df:
+            return (acc[0] + v,)
+        s, e = two_sum(acc[0], v)
+        return s, acc[1] + e
+
+    def comb(a, b):
+        if not df:
+            return (a[0] + b[0],)
+        s, e = two_sum(a[0], b[0])
+        e = e + (a[1] + b[1])
+        h = s + e
+        return h, e - (h - s)
+
+    def norm(a):
+        if not df:
+            return a
+        h = a[0] + a[1]
+        return h, a[1] - (h - a[0])
+
+    def zero(shape=()):
+        return tuple(np.zeros(shape, ft) for _ in range(2 if df else 1))
+
+    def ends(part):
+        acc = zero()
+        for v in lift(part):
+            acc = add(acc, v)
+        return norm(acc)
+
+    es = x.itemsize
+    vec = 16 // es
+    head = min((16 - off_bytes % 16) % 16 // es, x.size)
+    nvec = (x.size - head) // vec
+    body = lift(x[head:head + nvec * vec]).reshape(nvec, vec)
+    runs = -(-nvec // 512)
+    padded = np.zeros((runs * 512, vec), ft)
+    padded[:nvec] = body
+    real = (np.arange(runs * 512) < nvec).reshape(runs, 16, 32)
+    padded = padded.reshape(runs, 16, 32, vec)
+    accs = [zero((runs, 32)) for _ in range(chains)]
+    for j in range(16):
+        for e in range(vec):
+            new = add(accs[e % chains], padded[:, j, :, e])
+            accs[e % chains] = tuple(np.where(real[:, j], n, o) for n, o in zip(new, accs[e % chains]))
+    if chains == 4:
+        accs = [comb(accs[0], accs[1]), comb(accs[2], accs[3])]
+    lane = norm(comb(accs[0], accs[1]) if df else accs[0])
+    for m in (16, 8, 4, 2, 1):
+        lane = comb(lane, tuple(a[:, np.arange(32) ^ m] for a in lane))
+    slots = zero(512)
+    for s, a in zip(slots, lane):
+        s[:runs] = a[:, 0]
+    slots = comb(zero(512), slots)
+    w = 256
+    while w:
+        slots = comb(tuple(s[:w] for s in slots), tuple(s[w:2 * w] for s in slots))
+        w //= 2
+    total = comb(comb(ends(x[:head]), tuple(s[0] for s in slots)), ends(x[head + nvec * vec:]))
+    total = comb((ft(init), ft(0)) if df else (ft(init),), total)
+    return ft(total[0] + total[1]) if df else ft(total[0])
+
+
+@pytest.mark.parametrize("code", [C.F32, C.BF16, C.F64])
+def test_reduce_bits_follow_the_canonical_tree(dev, code):
+    """Sums of up to 32 runs (the one-block kernel) and of 33 to 70 (the kernel of
+    the long reduces), at starts on and off a 16-byte boundary: the bits of the
+    canonical tree restated in numpy."""
+    es = {C.F32: 4, C.BF16: 2, C.F64: 8}[code]
+    run = 8192 // es
+    rng = np.random.default_rng(code)
+    for n in (1, 16 // es, run - 1, run, 5 * run + 3, 31 * run + 7, 32 * run, 32 * run + 16 // es, 33 * run + 5, 70 * run):
+        for off in (0, 1):
+            x = rng.standard_normal(n) * np.exp(rng.standard_normal(n) * 4)
+            if code == C.BF16:
+                t = torch.from_numpy(x).to(torch.bfloat16)
+                bits = t.view(torch.int16).numpy().view(np.uint16)
+                ref = canonical_sum(bits, 0.5, 4, lambda b: (b.astype(np.uint32) << 16).view(np.float32), off * es)
+            else:
+                ft = np.float32 if code == C.F32 else np.float64
+                x = x.astype(ft)
+                t = torch.from_numpy(x)
+                ref = canonical_sum(x, 0.5, 2 if code == C.F32 else 1, lambda b: b, off * es)
+            base = torch.zeros(n + off, dtype=t.dtype, device="cuda")
+            base[off:] = t.cuda()
+            for cfg in (C.AUTO, 0, 47):
+                got = C.reduce(base[off:], "sum", init=0.5, config=cfg).cpu().numpy()[0]
+                assert got.tobytes() == ref.tobytes(), (n, off, cfg, got, ref)
