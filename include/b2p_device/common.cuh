@@ -40,8 +40,8 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void *p) {
   return r;
 }
 
-// The same through L2 only: for what a kernel that is still running when this
-// one starts may write (programmatic dependent launch, below).
+// The same as a coherent load, through L2: for what a kernel that is still
+// running when this one starts may write (programmatic dependent launch, below).
 __device__ __forceinline__ uint4 ld_stream_l2_v4(const void *p) {
   uint4 r;
   asm volatile("ld.global.cg.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -63,8 +63,9 @@ __device__ __forceinline__ void st_stream_v4(void *p, uint4 v) {
 // stream still runs.  It calls grid_wait() before its first access to global
 // memory (the kernels before it are complete and their writes visible then),
 // and grid_trigger() after that, so that no more than two kernels of a stream
-// overlap.  What an earlier kernel of the chain wrote is read through L2 only
-// (__ldcg, cp.async.cg): L1 is not invalidated in between.
+// overlap.  What an earlier kernel of the stream wrote is read by coherent
+// loads (plain ones, __ldcg, cp.async), never by .nc loads: the memory is not
+// read-only for the whole of such a kernel.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -13,7 +13,7 @@
 // Each digit pass (4 for 32-bit keys, 8 for 64-bit) is a reduce-then-scan
 // over persistent blocks, ping-ponging between the keys and a second array:
 //   * upsweep: block b counts the digits of its contiguous chunk of tiles
-//     (per-warp shared-memory counts), counts[d][b];
+//     (shared-memory counters by digit and lane), counts[d][b];
 //   * spine: per digit, an exclusive scan of its counts over the chunks and
 //     its total; a digit's first slot in chunk b is then the keys of smaller
 //     digits plus the keys of that digit in chunks before b;

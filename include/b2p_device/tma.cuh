@@ -56,18 +56,6 @@ __device__ __forceinline__ bool mbar_try(uint64_t *b, unsigned parity) {
   return ok != 0;
 }
 
-// Whether the phase has completed, without waiting.
-__device__ __forceinline__ bool mbar_test(uint64_t *b, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // try_wait with a suspend-time hint: the thread is parked (issues nothing)
 // until the phase completes or about `hint_ns` pass.  Waiting warps of the
 // pipelined kernels share their SM sub-partitions with the warps doing the
