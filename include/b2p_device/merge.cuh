@@ -470,34 +470,15 @@ __device__ __forceinline__ void merge_stage_chunk(T *slots, int c, const T *src,
   }
 }
 
-// Keys of sa[0..na) before output d of a staged tile: the first index that a
-// key of sb[0..nb) precedes, by binary lifting in steps of TOP, TOP / 2, ...
-// (the range is at most 2 TOP - 1 long).
-#pragma nv_exec_check_disable
-template <int TOP, class It, class Comp>
-__host__ __device__ __forceinline__ int merge_tile_split(It sa, It sb, int d, int na, int nb, const Comp &comp) {
-  int lo = d > nb ? d - nb : 0;
-  const int hi = d < na ? d : na;
-  It pa = sa + lo, pb = sb + (d - 1 - lo);
-#pragma unroll
-  for (int step = TOP; step > 0; step /= 2) {
-    if (lo + step <= hi && !comp(pb[1 - step], pa[step - 1])) {
-      lo += step;
-      pa += step;
-      pb -= step;
-    }
-  }
-  return lo;
-}
-
-// Whether ITEMS outputs that take ca keys of a, of which na are left, and
-// ITEMS - ca keys of b, of which nb are left, lie in the tile.  Always so when
-// both sides are in order.  Keys that are not, NaNs among others, can give
-// neighbouring threads splits that cross; such a thread merges serially, which
-// reads and writes keys of the tile whatever their order.
+// Whether the ITEMS outputs between two neighbouring splits, ca keys of a apart,
+// lie in the tile.  Always so when both sides are in order.  Keys that are not,
+// NaNs among others, can give splits that cross; such a thread merges serially,
+// which reads and writes keys of the tile whatever their order.  (Each split by
+// itself leaves no more keys of a side than there are, so that a ca from 0 to
+// ITEMS is enough.)
 template <int ITEMS>
-__host__ __device__ __forceinline__ bool merge_window_inside(int ca, int na, int nb) {
-  return ca >= 0 && ca <= ITEMS && ca <= na && ITEMS - ca <= nb;
+__host__ __device__ __forceinline__ bool merge_window_inside(int ca) {
+  return (unsigned)ca <= (unsigned)ITEMS;
 }
 
 // Persistent blocks: a block's next tile is on its way into the other buffer
@@ -558,9 +539,22 @@ __global__ void __launch_bounds__(MergeNet<T>::kThreads, MergeNet<T>::kBlocksPer
       range(tile + 2 * (long long)gridDim.x, i0, i1);
     }
     const int d = min(t * ITEMS, cnt);
-    constexpr int kTop = sizeof(T) == 4 ? 2048 : 1024;
-    static_assert(2 * kTop - 1 >= TILE / 2, "the steps reach every place");  // a range is TILE / 2 at most
-    const int lo = merge_tile_split<kTop>(sa, static_cast<const T *>(sb), d, na_t, nb_t, comp);
+    // keys of a before output d: the first in [lo, hi] that a key of b precedes
+    int lo = max(0, d - nb_t);
+    {
+      const int hi = min(d, na_t);  // hi - lo <= TILE / 2
+      constexpr int kTop = sizeof(T) == 4 ? 2048 : 1024;
+      static_assert(2 * kTop - 1 >= TILE / 2, "the steps reach every place");
+      const T *pa = sa + lo, *pb = sb + (d - 1 - lo);
+#pragma unroll
+      for (int step = kTop; step > 0; step /= 2) {
+        if (lo + step <= hi && !comp(pb[1 - step], pa[step - 1])) {
+          lo += step;
+          pa += step;
+          pb -= step;
+        }
+      }
+    }
     s_lo[t] = lo;
     if (t == 0) {
       s_lo[NT] = na_t;
@@ -569,7 +563,7 @@ __global__ void __launch_bounds__(MergeNet<T>::kThreads, MergeNet<T>::kBlocksPer
     __syncthreads();
     const int ca = s_lo[t + 1] - lo;
     T v[N];
-    bool serial = d + ITEMS > cnt || !merge_window_inside<ITEMS>(ca, na_t - lo, nb_t - (d - lo));
+    bool serial = d + ITEMS > cnt || !merge_window_inside<ITEMS>(ca);
     if (!serial) {
       const T *pa = sa + lo, *pb = sb + (d - lo + ITEMS);
 #pragma unroll

@@ -1,7 +1,7 @@
 // Steps of the device code that also compile for the host, run on the CPU:
 //   carries   the hand-over of a look-back unit's carries, with every slot
 //             taken again at the moment it is handed on;
-//   windows   the splits and windows of a merge tile whose keys are in order,
+//   windows   the windows between a merge tile's splits whose keys are in order,
 //             in no order, or have NaNs among them: every read inside the tile;
 //   counts    the keys that a merge tile takes of each range, for tile starts
 //             in order and crossing: never more than there are.
@@ -74,9 +74,20 @@ struct Checked {
   }
 };
 
-struct Before {
-  bool operator()(float x, float y) const { return x < y; }
-};
+// The split search of merge_keys_kernel: keys of sa[0..na) before output d.
+int tile_split(Checked sa, Checked sb, int d, int na, int nb) {
+  int lo = std::max(0, d - nb);
+  const int hi = std::min(d, na);
+  Checked pa = sa + lo, pb = sb + (d - 1 - lo);
+  for (int step = 2048; step > 0; step /= 2) {
+    if (lo + step <= hi && !(pb[1 - step] < pa[step - 1])) {
+      lo += step;
+      pa += step;
+      pb -= step;
+    }
+  }
+  return lo;
+}
 
 // One staged tile of fp32 keys: every thread's split, and the window of every
 // thread that merge_window_inside lets use the network (i < ca: key i of a,
@@ -90,11 +101,11 @@ void tile_windows(const std::vector<float> &a, const std::vector<float> &b, long
   b1.push_back(0.f);  // (the key after b's last)
   const Checked sa{a1.data(), 0, na, &outside}, sb{b1.data(), 0, nb, &outside};
   std::vector<int> lo(NT + 1, na);
-  for (int t = 0; t < NT; ++t) lo[t] = b2p::merge_tile_split<2048>(sa, sb, std::min(t * ITEMS, cnt), na, nb, Before{});
+  for (int t = 0; t < NT; ++t) lo[t] = tile_split(sa, sb, std::min(t * ITEMS, cnt), na, nb);
   for (int t = 0; t < NT; ++t) {
     const int d = std::min(t * ITEMS, cnt), ca = lo[t + 1] - lo[t];
     if (d + ITEMS > cnt) continue;
-    if (!b2p::merge_window_inside<ITEMS>(ca, na - lo[t], nb - (d - lo[t]))) {
+    if (!b2p::merge_window_inside<ITEMS>(ca)) {
       ++crossed;
       continue;
     }
