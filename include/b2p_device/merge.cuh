@@ -470,15 +470,14 @@ __device__ __forceinline__ void merge_stage_chunk(T *slots, int c, const T *src,
   }
 }
 
-// Whether the ITEMS outputs between two neighbouring splits, ca keys of a apart,
-// lie in the tile.  Always so when both sides are in order.  Keys that are not,
-// NaNs among others, can give splits that cross; such a thread merges serially,
-// which reads and writes keys of the tile whatever their order.  (Each split by
-// itself leaves no more keys of a side than there are, so that a ca from 0 to
-// ITEMS is enough.)
+// Keys of a among the ITEMS outputs between a thread's split and the next one's:
+// their difference when both sides are in order.  Keys that are not, NaNs among
+// others, can give splits that cross or lie more than ITEMS apart; the bounds then
+// keep the thread's keys inside the tile, for each split by itself leaves no
+// more keys of a side than there are.
 template <int ITEMS>
-__host__ __device__ __forceinline__ bool merge_window_inside(int ca) {
-  return (unsigned)ca <= (unsigned)ITEMS;
+__host__ __device__ __forceinline__ int merge_window(int lo, int next) {
+  return (int)min((unsigned)max(next, lo) - (unsigned)lo, (unsigned)ITEMS);
 }
 
 // Persistent blocks: a block's next tile is on its way into the other buffer
@@ -561,9 +560,9 @@ __global__ void __launch_bounds__(MergeNet<T>::kThreads, MergeNet<T>::kBlocksPer
       sb[nb_t] = K::last_key();
     }
     __syncthreads();
-    const int ca = s_lo[t + 1] - lo;
+    const int ca = merge_window<ITEMS>(lo, s_lo[t + 1]);
     T v[N];
-    bool serial = d + ITEMS > cnt || !merge_window_inside<ITEMS>(ca);
+    bool serial = d + ITEMS > cnt;
     if (!serial) {
       const T *pa = sa + lo, *pb = sb + (d - lo + ITEMS);
 #pragma unroll

@@ -89,9 +89,9 @@ int tile_split(Checked sa, Checked sb, int d, int na, int nb) {
   return lo;
 }
 
-// One staged tile of fp32 keys: every thread's split, and the window of every
-// thread that merge_window_inside lets use the network (i < ca: key i of a,
-// else key ITEMS - i of b, whose first one may be the key after b's last).
+// One staged tile of fp32 keys: every thread's split, and its window (i < ca:
+// key i of a, else key ITEMS - i of b, whose first one may be the key after b's
+// last).
 void tile_windows(const std::vector<float> &a, const std::vector<float> &b, long long &outside, int &crossed) {
   using Net = b2p::MergeNet<float>;
   constexpr int ITEMS = Net::kItems, NT = Net::kThreads;
@@ -103,12 +103,9 @@ void tile_windows(const std::vector<float> &a, const std::vector<float> &b, long
   std::vector<int> lo(NT + 1, na);
   for (int t = 0; t < NT; ++t) lo[t] = tile_split(sa, sb, std::min(t * ITEMS, cnt), na, nb);
   for (int t = 0; t < NT; ++t) {
-    const int d = std::min(t * ITEMS, cnt), ca = lo[t + 1] - lo[t];
+    const int d = std::min(t * ITEMS, cnt), ca = b2p::merge_window<ITEMS>(lo[t], lo[t + 1]);
     if (d + ITEMS > cnt) continue;
-    if (!b2p::merge_window_inside<ITEMS>(ca)) {
-      ++crossed;
-      continue;
-    }
+    crossed += ca != lo[t + 1] - lo[t];
     const Checked wa = sa + lo[t], wb{b1.data(), d - lo[t] + ITEMS, nb + 1, &outside};
     for (int i = 0; i <= ITEMS; ++i) (void)(i < ca ? wa + i : wb - i)[0];
   }
@@ -140,7 +137,7 @@ void windows() {
     }
     static const char *name[4] = {"windows, keys in order", "windows, keys in no order", "windows, NaNs at the end",
                                   "windows, NaNs anywhere"};
-    printf("(%d threads merge serially) ", crossed);
+    printf("(%d splits cross) ", crossed);
     check(outside == 0 && (kind == 0) == (crossed == 0), name[kind]);
   }
 }
