@@ -282,7 +282,9 @@ int b2p_segmented_per_call(int prim, int dtype, int op, const void *in, void *ou
 /* Stable merge of the sorted ranges a[0..na) and b[0..nb) into
  * out[0..na+nb) (ascending, or descending when descending != 0; on equal
  * keys the elements of a come first).  dtype I32, I64, U32, U64, F32, F64;
- * floats compare with < (NaNs unordered).  One pass: merge-path tiles.
+ * floats compare with < (NaNs unordered: the order of a result with NaNs is
+ * not specified, every key written is a key of a or b).  One pass:
+ * merge-path tiles.
  * scratch: device memory of at least b2p_scratch_bytes(B2P_PRIM_MERGE,
  * dtype, na + nb, 0, B2P_CONFIG_AUTO) bytes (the tile starts; no
  * initialisation needed, and like b2p_sort's not a look-back scratch
@@ -299,8 +301,9 @@ int b2p_merge(int dtype, const void *a, size_t na, const void *b, size_t nb, voi
  * second array of n keys and the merge passes' tile starts; its contents
  * need no initialisation).  The sort
  * overwrites it with keys, so it must not be a scratch buffer that the
- * other primitives use for their look-back status words.  A merge
- * sort: tiles sorted in shared memory, then log2(n / tile) merge passes.
+ * other primitives use for their look-back status words.  An LSD radix
+ * sort from 2^15 keys on; below, a merge sort: tiles sorted in shared
+ * memory, then log2(n / tile) merge passes (with NaNs as b2p_merge).
  * Replaces hipsycl::algorithms::sort (algorithms/algorithm.hpp:519-529,
  * algorithms/sort/bitonic_sort.hpp:69-110). */
 int b2p_sort(int dtype, void *keys, size_t n, int descending, void *scratch, size_t scratch_bytes,
@@ -390,7 +393,8 @@ typedef struct b2p_plan_s *b2p_plan;
  * inclusive scan (B2P_PRIM_SEG_SCAN) over fixed buffers, choose its launch
  * configuration (config or B2P_CONFIG_AUTO), allocate its scratch and
  * capture the launch into a CUDA graph on `stream`.  Blocks while it
- * captures.  The buffers must outlive the plan. */
+ * captures.  The buffers must outlive the plan; offsets in pageable host
+ * memory are copied and may go. */
 int b2p_plan_segmented(b2p_plan *plan, int prim, int dtype, int op,
                        const void *in, void *out, const int64_t *offsets,
                        int64_t nseg, size_t total_elems, int config,
